@@ -246,7 +246,8 @@ int configure_launch(qdfn_ctx* c) {
         if (const char* e = std::getenv("QDFN_SPEC_STOP")) c->spec_stop_pct = std::max(1, std::min(100, std::atoi(e)));
         int64_t want_chunks = std::max<int64_t>(1, (tiles_per_sm * sms + nrb - 1) / nrb);
         int64_t clen = (c->N + want_chunks - 1) / want_chunks;
-        // two x buffers (R x chunk x elem each) share the 227 KB with the 192 KB stage ring
+        // two x buffers (R x chunk x elem each) share the 227 KB with the 160 KB stage
+        // ring and the FP32 sums' pairs (8 KB per instance)
         const int64_t cmax = std::max<int64_t>(64, (int64_t)(15 * 1024) / (Rk * (int64_t)xsz));
         clen = (std::min<int64_t>(std::max<int64_t>(clen, 64), std::min<int64_t>(2048, cmax)) + 7) / 8 * 8;
         c->chunk_len = clen;
@@ -268,7 +269,8 @@ int configure_launch(qdfn_ctx* c) {
         // one x buffer: the chunk's columns rounded up to 4 (bulk copies move
         // multiples of 16 bytes), in 128-byte units
         c->xbuf = (((clen + 3) / 4 * 4) * Rk * (int64_t)xsz + 127) / 128 * 128 / (int64_t)xsz;
-        c->smem = (size_t)kPipeBytes + kMbarBytes + 2 * (size_t)c->xbuf * xsz;
+        c->smem = (size_t)kPipeBytes + kMbarBytes + 2 * (size_t)c->xbuf * xsz +
+                  (c->prec == QDFN_FP64 ? 0 : (size_t)Rk * fold_bytes<FmtF32, 1>());
         want_blocks = (nrb - nsmall) * c->nchunk + nsmall * c->nchunk2;
     }
     QDFN_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem));

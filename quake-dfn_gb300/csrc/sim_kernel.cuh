@@ -259,21 +259,29 @@ __device__ __forceinline__ void grid_fields(const double* slots_base, int nblk, 
 // ---------------------------------------------------------------------------
 // P2: dense elastic operator.
 //
-// Storage is tile-contiguous: receivers in row blocks of kSimThreads*VEC (one
-// 8-byte granule per thread and source column, 4 KB per column), and within a
+// Storage is tile-contiguous: receivers in row blocks of kOpThreads*VEC (one
+// 8-byte granule per thread and source column, 2 KB per column), and within a
 // row block the source columns back to back (see k_convert).  A tile is (row
 // block, chunk of source columns); tiles are handed out by a global counter.
-// Both matrices stream through a kStages-deep ring of 64 KB shared-memory
-// stages, each filled by one 32 KB TMA bulk copy per matrix
+// Both matrices stream through a kStages-deep ring of 32 KB shared-memory
+// stages (8 source columns), each filled by one 16 KB TMA bulk copy per matrix
 // (cp.async.bulk ... mbarrier::complete_tx) issued by one thread, so the bytes
 // in flight do not depend on the register-limited warp count of the
-// persistent kernel.  x = D (all R instances) is staged per tile.  FP32/BF16
-// products are summed in FP32 over 32 columns and folded error-free into
-// (hi, lo) FP32 pairs; FP64 storage accumulates in FP64.
+// persistent kernel.  That thread's own work per stage sets how soon a freed
+// slot is refilled, so a tile's geometry is worked out once per tile and a
+// stage costs it a wait, a descriptor, and two copies.  x = D (all R instances)
+// is staged per tile.  FP32/BF16 products are summed in FP32 over 32 columns
+// and folded error-free into (hi, lo) FP32 pairs, kept in shared memory between
+// folds; FP64 storage accumulates in FP64.
+// Measured against 64 KB stages with the pairs in registers (spilled) and the
+// geometry worked out per stage: 12,813 patches x 4, FP32, 20 steps 4529 ->
+// 4476 us; 40 networks x 4 in one launch, 15 steps 9411 -> 8468 us.  Four stages
+// instead of five: 1 % slower; stages of 16 columns with the pairs in registers
+// and this producer: 22 % slower.
 constexpr int kOpWarps = 8;                                     // operator role: warps [0, kOpWarps)
 constexpr int kOpThreads = kOpWarps * 32;
 constexpr int kProducerWarp = kSimThreads / 32 - 1;             // lane 0 fills the stage ring
-constexpr int kStages = 3;
+constexpr int kStages = 5;
 // FP32/BF16 steps that stream ahead: the solver warps [kOpWarps, kProducerWarp)
 // run the step's first reduction pass and its grid barrier on their own
 // (named barrier 1) while the operator warps and the producer finish the early
@@ -320,12 +328,12 @@ __device__ bool grid_barrier_solvers(const SimParams& p, uint64_t deadline_ns, u
     return s_ok != 0;
 }
 
-constexpr int kColsPerStage = 16;
+constexpr int kColsPerStage = 8;
 constexpr int kFoldStages = 32 / kColsPerStage;                 // FP32 sums span 32 columns
 constexpr int kSegBytes = kOpThreads * kGranule;                // one column of a row block, 2 KB
-constexpr int kStageBytes = 2 * kColsPerStage * kSegBytes;      // E and Kn, 64 KB
-constexpr int kPipeBytes = kStages * kStageBytes;               // 192 KB
-constexpr int kMbarBytes = 128;
+constexpr int kStageBytes = 2 * kColsPerStage * kSegBytes;      // E and Kn, 32 KB
+constexpr int kPipeBytes = kStages * kStageBytes;               // 160 KB
+constexpr int kMbarBytes = 256;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;                // 2 s per stage wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void* ptr) {
@@ -396,18 +404,21 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* m) {
 // Descriptor of the stage held by a ring slot.  The producer writes it before
 // the arrival that completes the slot's "full" barrier (release), consumers
 // read it after waiting on that barrier (acquire).
-struct StageDesc {
-    long long tile;   // operator tile, or -1: no tiles left (end marker)
+struct __align__(16) StageDesc {
+    int rb, c;        // operator tile: row block (-1: no tiles left, end marker) and column chunk
     int q, nst;       // stage index within the tile, stages of the tile
+    int nc;           // source columns of the stage
     int seq;          // tile sequence number in this CTA (selects the x buffer)
     int next;         // 1: a tile of the next step (streamed ahead)
+    int pad;
 };
-static_assert(6 * 8 + kStages * sizeof(StageDesc) <= kMbarBytes, "mbarriers + stage descriptors");
+constexpr int kDescOffset = (2 * 8 * kStages + 15) / 16 * 16;
+static_assert(kDescOffset + kStages * sizeof(StageDesc) <= kMbarBytes, "mbarriers + stage descriptors");
 
 // Pipeline state of one CTA: stage memory, the "full" mbarriers (completed by
 // the bulk copies' byte count), the "empty" mbarriers (one arrival per operator
 // warp once it has read the stage), the stage descriptors, and the running
-// stage counts.  `consumed` is identical in every operator thread; the
+// stage positions.  The consumers' is identical in every operator thread; the
 // producer fields are used by thread 0 alone.  The ring keeps running across
 // tiles (the producer walks into the next tile as soon as a slot frees up) and
 // across steps.
@@ -416,11 +427,13 @@ struct Pipe {
     uint64_t* full;
     uint64_t* empty;
     StageDesc* desc;
-    uint32_t consumed;
+    uint32_t cslot, cwrap;   // the next stage's slot and its round of the ring
     // producer (thread 0)
-    uint32_t filled;
+    uint32_t filled, fslot, fwrap;   // stages filled; the next one's slot and its round of the ring
     long long ftile;         // tile being filled; -2 none yet, -1 no tiles left
     int fq, fnst, fseq;      // its next stage, its stage count, its sequence number
+    int frb, fc, fj0, fleft; // its row block, column chunk, first column, columns not yet copied
+    int64_t foff;            // byte offset of its next stage in both matrices
     int fphase, fnext;       // 0 this step's tiles, 1 the next step's, 2 done; the tile's step
     uint32_t last_stage[2];  // last stage of the latest tile using each x buffer
 };
@@ -430,9 +443,9 @@ __device__ __forceinline__ void pipe_init(Pipe& pp, unsigned char* smem) {
     pp.stages = smem;
     pp.full = reinterpret_cast<uint64_t*>(smem + kPipeBytes);
     pp.empty = pp.full + kStages;
-    pp.desc = reinterpret_cast<StageDesc*>(pp.full + 2 * kStages);
-    pp.consumed = 0;
-    pp.filled = 0;
+    pp.desc = reinterpret_cast<StageDesc*>(smem + kPipeBytes + kDescOffset);
+    pp.cslot = pp.cwrap = 0;
+    pp.filled = pp.fslot = pp.fwrap = 0;
     pp.ftile = -2;
     pp.fq = pp.fnst = 0;
     pp.fseq = -1;
@@ -447,6 +460,15 @@ __device__ __forceinline__ void pipe_init(Pipe& pp, unsigned char* smem) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+}
+
+// Shared memory of the operator threads' (hi, lo) pairs (FP32/BF16 storage):
+// one float4 per receiver row and instance.  In registers they are 32 of a
+// thread's 128 for four instances and were spilled: at 6,400 patches x 4 the
+// local-memory traffic of the step was 0.75 of the operator's bytes.
+template <class M, int R>
+__host__ __device__ constexpr size_t fold_bytes() {
+    return sizeof(typename M::X) == 4 ? sizeof(float4) * (size_t)R * M::VEC * kOpThreads : 0;
 }
 
 // error-free accumulation of an FP32 partial sum into an unevaluated pair
@@ -756,10 +778,9 @@ __device__ __forceinline__ bool produce_stage(const SimParams& p, Pipe& pp, type
     constexpr int EB = kGranule / VEC;   // bytes per stored entry
     constexpr int64_t rows_per_blk = (int64_t)kOpThreads * VEC;
     const uint32_t n = pp.filled;
-    const int slot = (int)(n % kStages);
+    const int slot = (int)pp.fslot;
     // the stage this slot held last must be released by every operator warp
-    if (n >= (uint32_t)kStages && !mbar_wait(pp.empty + slot, ((n - kStages) / kStages) & 1u, kWaitLimitNs))
-        return false;
+    if (pp.fwrap > 0 && !mbar_wait(pp.empty + slot, (pp.fwrap - 1) & 1u, kWaitLimitNs)) return false;
     if (pp.ftile == -2 || (pp.ftile >= 0 && pp.fq >= pp.fnst)) {
         int64_t nrb_reg, n_spec;
         spec_shape(p, nrb, &nrb_reg, &n_spec);
@@ -806,21 +827,24 @@ __device__ __forceinline__ bool produce_stage(const SimParams& p, Pipe& pp, type
             pp.fnext = 1;
             break;
         }
-        if (pp.ftile >= 0) {
+        if (pp.ftile >= 0) {   // the tile's geometry, once per tile
+            const TileGeo g = tile_geo(p, nrb, pp.ftile);
             pp.fq = 0;
-            pp.fnst = tile_geo(p, nrb, pp.ftile).nst;
+            pp.fnst = g.nst;
             pp.fseq++;
+            pp.frb = g.rb; pp.fc = g.c; pp.fj0 = g.j0; pp.fleft = g.L;
+            pp.foff = (((int64_t)g.rb * p.N + g.j0) * rows_per_blk) * EB;
         }
     }
     StageDesc* d = pp.desc + slot;
     uint64_t* m = pp.full + slot;
+    pp.filled = n + 1;
+    if (++pp.fslot == (uint32_t)kStages) { pp.fslot = 0; ++pp.fwrap; }
     if (pp.ftile == -1) {              // end marker: completes the phase without bytes
-        d->tile = -1;
+        d->rb = -1;
         mbar_arrive(m);
-        pp.filled = n + 1;
         return true;
     }
-    const TileGeo g = tile_geo(p, nrb, pp.ftile);
     const int q = pp.fq;
     const int xb = pp.fseq & 1;
     if (q == 0) {
@@ -831,31 +855,28 @@ __device__ __forceinline__ bool produce_stage(const SimParams& p, Pipe& pp, type
             !mbar_wait(pp.empty + (prev % kStages), (prev / kStages) & 1u, kWaitLimitNs))
             return false;
     }
-    d->tile = pp.ftile;
-    d->q = q;
-    d->nst = g.nst;
-    d->seq = pp.fseq;
-    d->next = pp.fnext;
-    const int nc = (int)min((int64_t)kColsPerStage, g.L - (int64_t)q * kColsPerStage);
+    const int nc = min(kColsPerStage, pp.fleft);
+    reinterpret_cast<int4*>(d)[0] = make_int4(pp.frb, pp.fc, q, pp.fnst);
+    reinterpret_cast<int4*>(d)[1] = make_int4(nc, pp.fseq, pp.fnext, 0);
     const uint32_t bytes = (uint32_t)nc * kSegBytes;
     // x: the tile's columns rounded up to 4 (the copy is padded past N)
-    const uint32_t xbytes = q == 0 ? (uint32_t)(((g.L + 3) / 4 * 4) * R * sizeof(X)) : 0u;
+    const uint32_t xbytes = q == 0 ? (uint32_t)(((pp.fleft + 3) / 4 * 4) * R * sizeof(X)) : 0u;
     fence_proxy_async();
     mbar_expect_tx(m, 2u * bytes + xbytes);
     unsigned char* st = pp.stages + (size_t)slot * kStageBytes;
     // tile-contiguous layout: the nc columns of this row block are one run of
     // nc * kSegBytes in each matrix -> one bulk copy per matrix
-    const int64_t off = (((int64_t)g.rb * p.N + g.j0 + (int64_t)q * kColsPerStage) * rows_per_blk) * EB;
-    bulk_g2s(st, reinterpret_cast<const unsigned char*>(p.E) + off, bytes, m, pol);
-    bulk_g2s(st + (size_t)kColsPerStage * kSegBytes, reinterpret_cast<const unsigned char*>(p.Kn) + off, bytes, m,
+    bulk_g2s(st, reinterpret_cast<const unsigned char*>(p.E) + pp.foff, bytes, m, pol);
+    bulk_g2s(st + (size_t)kColsPerStage * kSegBytes, reinterpret_cast<const unsigned char*>(p.Kn) + pp.foff, bytes, m,
              pol);
     if (q == 0) {
         const X* xsrc = reinterpret_cast<const X*>(pp.fnext ? sc.xnext : sc.xcur);
-        bulk_g2s(xs + (size_t)xb * p.xbuf, xsrc + (int64_t)g.j0 * R, xbytes, m, pol);
+        bulk_g2s(xs + (size_t)xb * p.xbuf, xsrc + (int64_t)pp.fj0 * R, xbytes, m, pol);
     }
-    if (q == g.nst - 1) pp.last_stage[xb] = n;
+    if (q == pp.fnst - 1) pp.last_stage[xb] = n;
     pp.fq = q + 1;
-    pp.filled = n + 1;
+    pp.foff += bytes;
+    pp.fleft -= nc;
     return true;
 }
 
@@ -896,63 +917,78 @@ __device__ bool dense_matvec(const SimParams& p, Pipe& pp, typename M::X* xs, co
     constexpr int VEC = M::VEC;
     constexpr int64_t rows_per_blk = (int64_t)kOpThreads * VEC;
     const int64_t N = p.N;
-    const int64_t nrb = (N + rows_per_blk - 1) / rows_per_blk;
     bool ok = true;
     // FP64 storage: fs/fn are the accumulators.  FP32 storage: fs/fn sum
-    // kFoldStages stages, then fold error-free into the pairs (h, l).
+    // kFoldStages stages, then fold error-free into the pairs (hi, lo) of both
+    // matrices, which this thread keeps in shared memory (see fold_bytes)
     X fs[R][VEC], fn[R][VEC];
-    float hs[R][VEC], ls[R][VEC], hn[R][VEC], ln[R][VEC];
-    TileGeo g{};
+    float4* pairs = reinterpret_cast<float4*>(xs + 2 * p.xbuf) + threadIdx.x;
     int64_t i0 = 0;
     const X* xsb = xs;
     while (ok) {
-        const uint32_t n = pp.consumed;
-        const int slot = (int)(n % kStages);
-        if (!mbar_wait(pp.full + slot, (n / kStages) & 1u, kWaitLimitNs)) { ok = false; break; }
+        const int slot = (int)pp.cslot;
+        if (!mbar_wait(pp.full + slot, pp.cwrap & 1u, kWaitLimitNs)) { ok = false; break; }
         const StageDesc d = pp.desc[slot];
-        if (d.q == 0 && d.tile >= 0) {   // a new tile
-            g = tile_geo(p, nrb, d.tile);
-            i0 = (int64_t)g.rb * rows_per_blk + (int64_t)threadIdx.x * VEC;
+        if (d.q == 0 && d.rb >= 0) {   // a new tile
+            i0 = (int64_t)d.rb * rows_per_blk + (int64_t)threadIdx.x * VEC;
             xsb = xs + (size_t)(d.seq & 1) * p.xbuf;
 #pragma unroll
             for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int v = 0; v < VEC; ++v) {
-                    fs[r][v] = 0; fn[r][v] = 0;
-                    hs[r][v] = 0.f; ls[r][v] = 0.f; hn[r][v] = 0.f; ln[r][v] = 0.f;
-                }
+                for (int v = 0; v < VEC; ++v) { fs[r][v] = 0; fn[r][v] = 0; }
         }
-        if (d.tile >= 0 && i0 < N) {
-            const int q = d.q;
-            const int nc = (int)min((int64_t)kColsPerStage, g.L - (int64_t)q * kColsPerStage);
+        if (d.rb >= 0 && i0 < N) {
+            const int q = d.q, nc = d.nc;
             const unsigned char* st = pp.stages + (size_t)slot * kStageBytes + (size_t)threadIdx.x * kGranule;
+            const X* xq = xsb + (int64_t)q * kColsPerStage * R;
+            auto column = [&](int cc) {
+                X e[VEC], k[VEC], x[R];
+                M::sload(st + (size_t)cc * kSegBytes, e);
+                M::sload(st + (size_t)(kColsPerStage + cc) * kSegBytes, k);
+                xload<X, R>(xq + cc * R, x);
 #pragma unroll
-            for (int cc = 0; cc < kColsPerStage; ++cc) {
-                if (cc < nc) {
-                    X e[VEC], k[VEC], x[R];
-                    M::sload(st + (size_t)cc * kSegBytes, e);
-                    M::sload(st + (size_t)(kColsPerStage + cc) * kSegBytes, k);
-                    xload<X, R>(xsb + ((int64_t)q * kColsPerStage + cc) * R, x);
+                for (int r = 0; r < R; ++r)
 #pragma unroll
-                    for (int r = 0; r < R; ++r)
-#pragma unroll
-                        for (int v = 0; v < VEC; ++v) {
-                            fs[r][v] = fma(e[v], x[r], fs[r][v]);
-                            fn[r][v] = fma(k[v], x[r], fn[r][v]);
-                        }
-                }
+                    for (int v = 0; v < VEC; ++v) {
+                        fs[r][v] = fma(e[v], x[r], fs[r][v]);
+                        fn[r][v] = fma(k[v], x[r], fn[r][v]);
+                    }
+            };
+            if (nc == kColsPerStage) {
+#pragma unroll 16
+                for (int cc = 0; cc < kColsPerStage; ++cc) column(cc);
+            } else {
+#pragma unroll 1
+                for (int cc = 0; cc < nc; ++cc) column(cc);
             }
+            // the tile's partials go to its step's buffer
+            const bool last = q == d.nst - 1;
+            const int64_t o0 = (int64_t)(sc.ppar ^ d.next) * p.part_stride + (int64_t)d.c * R * N + i0;
             if constexpr (sizeof(X) == 4) {
-                if ((q + 1) % kFoldStages == 0 || q == d.nst - 1) {
+                if ((q + 1) % kFoldStages == 0 || last) {
 #pragma unroll
                     for (int r = 0; r < R; ++r)
 #pragma unroll
                         for (int v = 0; v < VEC; ++v) {
-                            two_sum_acc(hs[r][v], ls[r][v], (float)fs[r][v]);
-                            two_sum_acc(hn[r][v], ln[r][v], (float)fn[r][v]);
+                            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);   // (hi, lo) of E, of Kn
+                            if (q >= kFoldStages) a = pairs[(r * VEC + v) * kOpThreads];
+                            two_sum_acc(a.x, a.y, (float)fs[r][v]);
+                            two_sum_acc(a.z, a.w, (float)fn[r][v]);
                             fs[r][v] = 0;
                             fn[r][v] = 0;
+                            if (!last) {
+                                pairs[(r * VEC + v) * kOpThreads] = a;
+                            } else if (i0 + v < N) {   // the pair itself: no FP64 work in this phase
+                                reinterpret_cast<float2*>(p.part_s)[o0 + r * N + v] = make_float2(a.x, a.y);
+                                reinterpret_cast<float2*>(p.part_n)[o0 + r * N + v] = make_float2(a.z, a.w);
+                            }
                         }
+                }
+            } else if (last) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    p.part_s[o0 + r * N] = fs[r][0];
+                    p.part_n[o0 + r * N] = fn[r][0];
                 }
             }
         }
@@ -960,35 +996,15 @@ __device__ bool dense_matvec(const SimParams& p, Pipe& pp, typename M::X* xs, co
         // every warp has arrived, the other warps run ahead into filled stages
         __syncwarp();
         if ((threadIdx.x & 31) == 0) mbar_arrive(pp.empty + slot);
-        pp.consumed = n + 1;
-        if (d.tile < 0) break;             // end marker
-        if (d.q == d.nst - 1) {            // the tile is complete: partials, then publish
-            if (i0 < N) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-#pragma unroll
-                    for (int v = 0; v < VEC; ++v) {
-                        const int64_t i = i0 + v;
-                        if (i < N) {
-                            // the tile's step selects the partial buffer
-                            const int64_t o = (int64_t)(sc.ppar ^ d.next) * p.part_stride +
-                                              ((int64_t)g.c * R + r) * N + i;
-                            if constexpr (sizeof(X) == 8) {
-                                p.part_s[o] = fs[r][v];
-                                p.part_n[o] = fn[r][v];
-                            } else {   // the pair itself: no FP64 work in this phase
-                                reinterpret_cast<float2*>(p.part_s)[o] = make_float2(hs[r][v], ls[r][v]);
-                                reinterpret_cast<float2*>(p.part_n)[o] = make_float2(hn[r][v], ln[r][v]);
-                            }
-                        }
-                    }
-            }
+        if (++pp.cslot == (uint32_t)kStages) { pp.cslot = 0; ++pp.cwrap; }
+        if (d.rb < 0) break;               // end marker
+        if (d.q == d.nst - 1) {            // the tile is complete: publish its partials
             __threadfence();
             __syncwarp();
             if ((threadIdx.x & 31) == 0) {
-                const unsigned old = atomicAdd(p.rb_done + (d.next ? sc.set_next : sc.set) * p.rb_stride + g.rb, 1u);
+                const unsigned old = atomicAdd(p.rb_done + (d.next ? sc.set_next : sc.set) * p.rb_stride + d.rb, 1u);
                 // diagnostics: when the step's last row block became complete
-                if (!d.next && sc.t0 != 0 && old + 1 == (unsigned)chunks_of_rb(p, g.rb) * kOpWarps)
+                if (!d.next && sc.t0 != 0 && old + 1 == (unsigned)chunks_of_rb(p, d.rb) * kOpWarps)
                     atomicMax(p.tmax + sc.set * 4 + 3, (unsigned long long)(globaltimer_ns() - sc.t0));
             }
         }
