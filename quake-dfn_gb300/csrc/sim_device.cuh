@@ -14,6 +14,7 @@
 // Dt < 1e-10 in the high-V solver) the device code continues as if the user
 // pressed Enter.
 #pragma once
+#include "friction_math.cuh"
 #include "qdfn_internal.h"
 
 namespace qdfn {
@@ -341,6 +342,75 @@ static __device__ PatchOut solve_highv_pair(const PatchIn& p, double Dt, double 
         else { Dt = Dt / 2; QDFN_RESET(); maxDiff = 0; FLAG = 0; }   \
     } while (0)
 
+// Newton iteration for the low-velocity step, for the usual case: the aging
+// law with Alpha_Evo = 0 and operands of ordinary size.  It solves the same
+// equation as solve_lowv below to the same tolerance.  With u = V - VOld the
+// friction is linear, mu(V) = Fb - g u, and ln(V0 Theta / Dc) = L0 - ln(1 + q V)
+// with q = Dt / Dc, so the residual needs one logarithm and one exponential per
+// iteration:
+//   f(V) = V - V0 exp(c0 - (g/a) u + (b/a) ln(1 + q V)),
+//   c0 = (Fb - F0 - b L0) / a,
+// and the slope comes in closed form, where the secant rule evaluates the
+// residual a second time at V (1 + 1e-10) and gets the slope with a relative
+// noise of 1e-5..1e-4 from the rounding of the two values.  The slope only has
+// to make the iteration contract, so it is formed in FP32 (relative error
+// ~1e-6), as is the step f / slope; V, the residual and the outputs are FP64.
+// A step below 1e-9 V ends the iteration, as in the reference (|VTest/V - 1|),
+// with an error of that step times the slope's error.
+// Returns false -- nothing decided -- when an operand or an iterate leaves the
+// ordinary range (V in (1e-25, 1e3), |ln(V/V0)| < 60) or 16 iterations are not
+// enough: the caller then runs the reference loop from the start, with all its
+// branches.
+// The solves are bound by the FP64 pipe (a warp instruction per 16 clocks and
+// SM) and the chain of dependent FP64 operations: ~120 of them per solve here,
+// ~620 in the secant loop.  Measured alone, 1 M patches on every SM: 1.41 ->
+// 0.29 ns a solve, largest error of V against an extended-precision root
+// 1.7e-13 -> 2.7e-14.  In the step (both sides with the present operator
+// stream): 40 networks x 4 draws in one launch, 15 steps 8525 -> 4585 us; 800
+// patches FP64 through `main` 16.1 -> 11.8 ms; a 6,000-triangle H-matrix run
+// 2232 -> 1704 us.
+__device__ __forceinline__ bool hi_between(double x, double lo, double hi) {   // 0 < lo <= x < hi, NaN excluded
+    return (unsigned)(__double2hiint(x) - __double2hiint(lo)) < (unsigned)(__double2hiint(hi) - __double2hiint(lo));
+}
+__device__ __forceinline__ bool solve_lowv_newton(const PatchIn& p, double Dt, double eta, double alpha, int dr,
+                                                  PatchOut& o) {
+    const double th = p.ThetaOld + Dt;
+    const bool usual = dr == 1 && (__double_as_longlong(alpha) << 1) == 0 && hi_between(p.VOld, 1e-25, 1e3) &&
+                       hi_between(p.sigma, 1e-20, 1e20) && hi_between(fabs(p.sigma_old), 1e-20, 1e20) &&
+                       hi_between(p.a, 1e-9, 1e9) && hi_between(fabs(p.b), 1e-9, 1e9) &&
+                       hi_between(p.Dc, 1e-12, 1e12) && hi_between(Dt, 1e-14, 1e14) && hi_between(th, 1e-20, 1e25);
+    if (!usual) return false;
+    const double inv_sig = 1 / p.sigma;
+    const double Fb = inv_sig * (p.K_Self * (p.TLD - fma(p.VOld, Dt, p.DispOld)) + p.tau0 - eta * p.VOld + p.dtau);
+    const double g = inv_sig * (fma(p.K_Self, 0.5 * Dt, eta) + p.Mass * p.rDt);
+    const double q = Dt * p.rDc, ga = g * p.ra, ba = p.b * p.ra;
+    const double c0 = (Fb - p.Friction0 - p.b * fm_log(th * (kV0 * p.rDc))) * p.ra;
+    const float gaf = (float)ga, bqf = (float)ba * (float)q, qf = (float)q;
+    double V = p.VOld;
+    float Vf = (float)V;
+    int it = 0;
+    for (;;) {
+        ++it;
+        const double x = fma(ba, fm_log(fma(V, q, 1.0)), fma(-ga, V - p.VOld, c0));
+        if (!((unsigned)(__double2hiint(x) & 0x7fffffff) < (unsigned)__double2hiint(60.0))) return false;
+        const double e = fm_exp(x);
+        const float f = (float)fma(-kV0, e, V);
+        const float slope = fmaf((float)kV0 * (float)e, gaf - __fdividef(bqf, fmaf(Vf, qf, 1.f)), 1.f);
+        const float d = __fdividef(f, slope);
+        V -= (double)d;
+        if (!hi_between(V, 1e-25, 1e3)) return false;
+        Vf = (float)V;
+        if (fabsf(d) <= 1e-9f * Vf) break;
+        if (it == 16) return false;
+    }
+    o.V = V;
+    o.Friction = fma(-g, V - p.VOld, Fb);
+    o.Disp = p.DispOld + (p.VOld + V) * 0.5 * Dt;
+    o.Theta = th / fma(V, q, 1.0);
+    o.Dt = Dt; o.Instab = 0; o.Flag = 1; o.Iterations = it;
+    return hi_between(fabs(o.Friction), 1e-300, 1e300) || o.Friction == 0.0;
+}
+
 // One lane per patch.
 static __device__ PatchOut solve_lowv(const PatchIn& p, double Dt, double eta, double alpha, int dr,
                                double SwitchV, int& err) {
@@ -497,6 +567,18 @@ static __device__ PatchOut solve_lowv_pair(const PatchIn& p, double Dt, double e
 #undef QDFN_THETA_NAN
 #undef QDFN_ITER_CAP
 #undef QDFN_RESET
+
+// The reference loops, one lane or a lane pair per patch, for what
+// solve_lowv_newton leaves.  Inlined: a call from the persistent kernel makes
+// the operator warps save their sums around it (12,813 patches x 4: 3.3 times
+// slower).  `in` is a copy, so that the caller's operands stay in registers.
+static __device__ __forceinline__ PatchOut solve_reference(PatchIn in, bool high, bool pair, double Dt, double eta,
+                                                        double alpha, int dr, double SwitchV, int& err) {
+    if (high)
+        return pair ? solve_highv_pair(in, Dt, eta, alpha, dr, err) : solve_highv(in, Dt, eta, alpha, dr, err);
+    return pair ? solve_lowv_pair(in, Dt, eta, alpha, dr, SwitchV, err)
+                : solve_lowv(in, Dt, eta, alpha, dr, SwitchV, err);
+}
 
 // InterpolateFromStressChange for one patch column.
 __device__ __forceinline__ void interp_ext(int64_t nt, const double* __restrict__ t,

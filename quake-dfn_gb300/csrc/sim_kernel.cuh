@@ -1293,14 +1293,8 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                 int err = 0;
                 sim::PatchOut o;
                 const int swq = QDFN_CUR(sw, sw_n)[q];
-                if (swq == 1) {
-                    o = pair ? sim::solve_highv_pair(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, err)
-                             : sim::solve_highv(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, err);
-                } else if (pair) {
-                    o = sim::solve_lowv_pair(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, p.switch_v, err);
-                } else {
-                    o = sim::solve_lowv(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, p.switch_v, err);
-                }
+                if (swq == 1 || !sim::solve_lowv_newton(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, o))
+                    o = sim::solve_reference(pin, swq == 1, pair, Dt, p.eta, p.alpha_evo, p.evolution_dr, p.switch_v, err);
                 if (!writer) return;
                 if (p.sw_used) p.sw_used[q] = (unsigned char)swq;
                 QDFN_NXT(V, Vn)[q] = o.V; QDFN_NXT(fric, fn)[q] = o.Friction; QDFN_NXT(D, Dn)[q] = o.Disp;
