@@ -55,8 +55,7 @@ extern "C" int qdfn_assemble_rect_dev(int64_t n_src, const double* src, int64_t 
     if (rc) return rc;
     if (n_src == 0 || n_recv == 0) return QDFN_OK;
     if (!src || !recv || !Ks || !Kn) return fail(QDFN_ERR_INVALID, "null pointer");
-    launch_assemble_rect(asm_grid(n_src, n_recv), (cudaStream_t)stream, n_src, src, n_recv, recv,
-                         G, nu, Ks, Kn, ld, layout);
+    launch_assemble_rect((cudaStream_t)stream, n_src, src, n_recv, recv, G, nu, Ks, Kn, ld, layout);
     QDFN_CUDA(cudaGetLastError());
     return QDFN_OK;
 }
