@@ -19,12 +19,6 @@
 namespace qdfn {
 namespace {
 
-dim3 asm_grid(int64_t n_src, int64_t n_recv) {
-    int64_t gx = (n_recv + kAsmThreads - 1) / kAsmThreads;
-    int64_t gy = n_src < 65535 ? n_src : 65535;
-    return dim3((unsigned)gx, (unsigned)(gy > 0 ? gy : 1), 1);
-}
-
 int check_common(int64_t n_src, int64_t n_recv, int64_t ld, int layout) {
     if (n_src < 0 || n_recv < 0) return fail(QDFN_ERR_INVALID, "negative patch count");
     if (layout != QDFN_LAYOUT_ROW && layout != QDFN_LAYOUT_COL)
@@ -93,7 +87,7 @@ extern "C" int qdfn_assemble_tri_dev(int64_t n_src, const double* P1, const doub
     if (n_src == 0 || n_recv == 0) return QDFN_OK;
     if (!P1 || !P2 || !P3 || !rake || !centre || !nhat || !shat || !Ks || !Kn)
         return fail(QDFN_ERR_INVALID, "null pointer");
-    launch_assemble_tri(asm_grid(n_src, n_recv), (cudaStream_t)stream, n_src, P1, P2, P3, rake,
+    launch_assemble_tri((cudaStream_t)stream, n_src, P1, P2, P3, rake,
                         n_recv, centre, nhat, shat, G, nu, Ks, Kn, ld, layout);
     QDFN_CUDA(cudaGetLastError());
     return QDFN_OK;
