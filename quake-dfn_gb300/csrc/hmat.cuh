@@ -164,9 +164,11 @@ __device__ __forceinline__ BlkA load_blk_a(const Blk* p) {
 // rows_a rank rows): the lanes stride the block's source range, each load of
 // x serving every row of the group, and each round issues the group's rows x 4
 // column loads before any of them is used (HBM latency is hidden by the loads
-// in flight, not by occupancy: one 16-warp CTA per SM)
+// in flight, not by occupancy: one 16-warp CTA per SM).  Out of line, like pass
+// B: beside the inlined solvers the loops lost registers and loads in flight
+// (6,000 triangles: the two passes 51 us a step, 42 out of line).
 template <class T, int R>
-__device__ void pass_a(const Ops& h, const double* __restrict__ D, int64_t N, T*, double*) {
+__device__ __noinline__ void pass_a(const Ops h, const double* __restrict__ D, int64_t N, T*, double*) {
     constexpr int G = rows_a<R>();
     // 32-column rounds per batch (G x kUA loads per lane in flight), within the
     // persistent kernel's 128 registers
@@ -325,7 +327,7 @@ __device__ void pass_b_range(const Ops& h, const double* __restrict__ D, int64_t
 // wait (pass A ran in an earlier launch).  Returns false if the wait gave up
 // (limit_ns, or another block's error in *gerr).
 template <class T, int R>
-__device__ bool pass_b(const Ops& h, const double* __restrict__ D, int64_t N, unsigned long long a_target,
+__device__ __noinline__ bool pass_b(const Ops h, const double* __restrict__ D, int64_t N, unsigned long long a_target,
                        uint64_t limit_ns, const int* gerr) {
     pass_b_range<T, R>(h, D, N, 0, h.n_tiles_dense);
     if (h.n_tiles <= h.n_tiles_dense) return true;

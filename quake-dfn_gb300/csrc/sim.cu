@@ -141,7 +141,7 @@ SimParams make_params(qdfn_ctx* c, uint64_t budget_ns) {
     p.rowsum_n = offs ? c->rowsum_n : nullptr;
     p.evolution_dr = c->prob.evolution_dr; p.interp_at_told = c->prob.interp_at_told; p.hmat = c->hmat;
     p.eta = c->eta; p.sigma_min = c->prob.sigma_min; p.switch_v = c->prob.switch_v;
-    p.dt_cut = c->prob.dt_cut; p.rupture_dt = c->prob.rupture_dt; p.max_dt = c->prob.max_dt;
+    p.dt_cut = c->prob.dt_cut; p.r_dt_cut = 1.0 / c->prob.dt_cut; p.rupture_dt = c->prob.rupture_dt; p.max_dt = c->prob.max_dt;
     p.alpha_evo = c->prob.alpha_evo;
     p.record_step = c->prob.record_step; p.max_records = c->prob.max_records;
     p.a = c->a; p.b = c->b; p.Dc = c->Dc; p.F0 = c->F0; p.tau0 = c->tau0; p.sigma0 = c->sigma0;
@@ -249,7 +249,11 @@ int configure_launch(qdfn_ctx* c) {
         // two x buffers (R x chunk x elem each) share the 227 KB with the 160 KB stage
         // ring and the FP32 sums' pairs (8 KB per instance)
         const int64_t cmax = std::max<int64_t>(64, (int64_t)(15 * 1024) / (Rk * (int64_t)xsz));
-        clen = (std::min<int64_t>(std::max<int64_t>(clen, 64), std::min<int64_t>(2048, cmax)) + 7) / 8 * 8;
+        // at least 64 columns, 32 in FP64: its tiles take the FP64 pipe 32 times an
+        // FP32 tile's time, so small systems spread them over more blocks (800
+        // patches: 52 tiles on 25 blocks 25 us a step, 100 on 100)
+        const int64_t cmin = c->prec == QDFN_FP64 ? 32 : 64;
+        clen = (std::min<int64_t>(std::max<int64_t>(clen, cmin), std::min<int64_t>(2048, cmax)) + 7) / 8 * 8;
         c->chunk_len = clen;
         c->nchunk = (int)((c->N + clen - 1) / clen);
         // the row blocks of the last two waves of tiles are streamed by their own
@@ -277,9 +281,9 @@ int configure_launch(qdfn_ctx* c) {
     int occ = 0;
     QDFN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kSimThreads, c->smem));
     if (occ < 1) return fail(QDFN_ERR_CUDA, "simulation kernel cannot be resident");
-    const int64_t work_items = (int64_t)Rk * c->N;
+    // a block per tile, up to the SMs -- also where that leaves a block less than
+    // a warp of patch solves, which take a warp's time whether it is full or not
     int64_t nb = std::min<int64_t>((int64_t)sms * occ, std::max<int64_t>(1, want_blocks));
-    nb = std::max<int64_t>(1, std::min<int64_t>(nb, std::max<int64_t>((work_items + 31) / 32, 1)));
     if (c->nblocks_override > 0) nb = std::min<int64_t>(nb, c->nblocks_override);
     c->nblocks = (int)nb;
     if (c->hmat) {

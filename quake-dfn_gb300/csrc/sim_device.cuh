@@ -352,9 +352,12 @@ static __device__ PatchOut solve_highv_pair(const PatchIn& p, double Dt, double 
 //   c0 = (Fb - F0 - b L0) / a,
 // and the slope comes in closed form, where the secant rule evaluates the
 // residual a second time at V (1 + 1e-10) and gets the slope with a relative
-// noise of 1e-5..1e-4 from the rounding of the two values.  The slope only has
-// to make the iteration contract, so it is formed in FP32 (relative error
-// ~1e-6), as is the step f / slope; V, the residual and the outputs are FP64.
+// noise of 1e-5..1e-4 from the rounding of the two values: the iterates are the
+// secant rule's up to that noise.  (They have to be.  With b > a and a long step
+// the equation has several roots, and a step of higher order -- Halley's was
+// tried -- reaches another one than the reference's.)  The slope only has to
+// make the iteration contract, so it is formed in FP32 (relative error ~1e-6),
+// as is the step f / slope; V, the residual and the outputs are FP64.
 // A step below 1e-9 V ends the iteration, as in the reference (|VTest/V - 1|),
 // with an error of that step times the slope's error.
 // Returns false -- nothing decided -- when an operand or an iterate leaves the
@@ -362,9 +365,9 @@ static __device__ PatchOut solve_highv_pair(const PatchIn& p, double Dt, double 
 // enough: the caller then runs the reference loop from the start, with all its
 // branches.
 // The solves are bound by the FP64 pipe (a warp instruction per 16 clocks and
-// SM) and the chain of dependent FP64 operations: ~120 of them per solve here,
+// SM) and the chain of dependent FP64 operations: ~110 of them per solve here,
 // ~620 in the secant loop.  Measured alone, 1 M patches on every SM: 1.41 ->
-// 0.29 ns a solve, largest error of V against an extended-precision root
+// 0.20 ns a solve (0.25 with conversion instructions and IEEE divisions), largest error of V against an extended-precision root
 // 1.7e-13 -> 2.7e-14.  In the step (both sides with the present operator
 // stream): 40 networks x 4 draws in one launch, 15 steps 8525 -> 4585 us; 800
 // patches FP64 through `main` 16.1 -> 11.8 ms; a 6,000-triangle H-matrix run
@@ -380,33 +383,34 @@ __device__ __forceinline__ bool solve_lowv_newton(const PatchIn& p, double Dt, d
                        hi_between(p.a, 1e-9, 1e9) && hi_between(fabs(p.b), 1e-9, 1e9) &&
                        hi_between(p.Dc, 1e-12, 1e12) && hi_between(Dt, 1e-14, 1e14) && hi_between(th, 1e-20, 1e25);
     if (!usual) return false;
-    const double inv_sig = 1 / p.sigma;
+    const double inv_sig = fm_rcp(p.sigma);
     const double Fb = inv_sig * (p.K_Self * (p.TLD - fma(p.VOld, Dt, p.DispOld)) + p.tau0 - eta * p.VOld + p.dtau);
     const double g = inv_sig * (fma(p.K_Self, 0.5 * Dt, eta) + p.Mass * p.rDt);
     const double q = Dt * p.rDc, ga = g * p.ra, ba = p.b * p.ra;
     const double c0 = (Fb - p.Friction0 - p.b * fm_log(th * (kV0 * p.rDc))) * p.ra;
-    const float gaf = (float)ga, bqf = (float)ba * (float)q, qf = (float)q;
+    const float gaf = to_float(ga), qf = to_float(q), bqf = to_float(ba) * qf;
     double V = p.VOld;
-    float Vf = (float)V;
+    float Vf = to_float(V);
     int it = 0;
     for (;;) {
         ++it;
         const double x = fma(ba, fm_log(fma(V, q, 1.0)), fma(-ga, V - p.VOld, c0));
         if (!((unsigned)(__double2hiint(x) & 0x7fffffff) < (unsigned)__double2hiint(60.0))) return false;
         const double e = fm_exp(x);
-        const float f = (float)fma(-kV0, e, V);
-        const float slope = fmaf((float)kV0 * (float)e, gaf - __fdividef(bqf, fmaf(Vf, qf, 1.f)), 1.f);
+        const float f = to_float(fma(-kV0, e, V));
+        const float slope = fmaf((float)kV0 * to_float(e), gaf - __fdividef(bqf, fmaf(Vf, qf, 1.f)), 1.f);
         const float d = __fdividef(f, slope);
-        V -= (double)d;
+        V -= to_double(d);
         if (!hi_between(V, 1e-25, 1e3)) return false;
-        Vf = (float)V;
+        Vf = to_float(V);
         if (fabsf(d) <= 1e-9f * Vf) break;
         if (it == 16) return false;
     }
     o.V = V;
     o.Friction = fma(-g, V - p.VOld, Fb);
     o.Disp = p.DispOld + (p.VOld + V) * 0.5 * Dt;
-    o.Theta = th / fma(V, q, 1.0);
+    const double den = fma(V, q, 1.0), iden = fm_rcp(den), thn = th * iden;
+    o.Theta = fma(fma(-thn, den, th), iden, thn);
     o.Dt = Dt; o.Instab = 0; o.Flag = 1; o.Iterations = it;
     return hi_between(fabs(o.Friction), 1e-300, 1e300) || o.Friction == 0.0;
 }
@@ -568,8 +572,76 @@ static __device__ PatchOut solve_lowv_pair(const PatchIn& p, double Dt, double e
 #undef QDFN_ITER_CAP
 #undef QDFN_RESET
 
+// The high-velocity secant loop for the usual case (as solve_lowv_newton:
+// ordinary operands, aging law, Alpha_Evo = 0), point for point the reference's
+// -- the same secant rule with DV = VOld / 100 from V = VOld / 1e10, the same stop
+// -- with the oscillator map evaluated in fewer operations:
+//   W(V) = A0 - B (a ln(V/V0) + b ln(V0 Theta / Dc) + eta V / sigma),
+//   Theta = (ThetaOld - Dc/V) exp(-V Dt/Dc) + Dc/V,
+// where A0 and B hold what stays fixed in the solve.  The slope is not in closed
+// form here: the rule's coarse DV decides which root it goes to, so its points
+// are kept.  One evaluation is a chain of ~45 FP64 operations (two logarithms
+// side by side, an exponential, a reciprocal) instead of ~120, and a solve of
+// nine iterations has eighteen.  False -- nothing decided -- when a point leaves
+// the ordinary range or 98 iterations are not enough (the reference halves Dt
+// from the 100th on).
+// Measured: 4,005 patches, 200 of them on this solver, FP64, 20 steps 4337 -> 2803
+// us; 800 patches through `main`, a few such solves in 200 steps, 9.3 -> 8.4 ms.
+__device__ __forceinline__ bool solve_highv_usual(const PatchIn& p, double Dt, double eta, double alpha, int dr,
+                                                  PatchOut& o) {
+    const bool usual = dr == 1 && (__double_as_longlong(alpha) << 1) == 0 && hi_between(p.VOld, 1e-15, 1e4) &&
+                       hi_between(p.sigma, 1e-20, 1e20) && hi_between(fabs(p.sigma_old), 1e-20, 1e20) &&
+                       hi_between(p.a, 1e-9, 1e9) && hi_between(fabs(p.b), 1e-9, 1e9) &&
+                       hi_between(p.Dc, 1e-12, 1e12) && hi_between(Dt, 1e-14, 1e14) &&
+                       hi_between(p.ThetaOld, 1e-25, 1e25) && hi_between(p.K_Self, 1e-20, 1e30) &&
+                       hi_between(p.Omega, 1e-20, 1e20);
+    if (!usual) return false;
+    const double cO = cos(p.Omega * Dt), sO = sin(p.Omega * Dt);
+    const double iK = fm_rcp(p.K_Self), rDt2 = 2.0 * p.rDt;
+    // D(V) - DispOld = (DispOld - F)(cO - 1) + (VOld / Omega) sO,
+    // F = TLD + (tau0 + dtau - sigma (F0 + ...) - eta V) / K
+    const double w = (1.0 - cO) * rDt2;
+    const double F0 = p.TLD + (p.tau0 + p.dtau - p.sigma * p.Friction0) * iK;
+    const double A0 = fma(w, F0 - p.DispOld, fma(p.VOld * fm_rcp(p.Omega) * sO, rDt2, -p.VOld));
+    const double Ba = w * iK * p.sigma, qn = -Dt * p.rDc, kth = kV0 * p.rDc, Be = w * iK * eta;
+    const double Baa = -Ba * p.a, Bab = -Ba * p.b;
+    // W at V, the state and the two logarithms there; false out of range
+    auto eval = [&](double V, double& Th, double& lv, double& lt, double& W) {
+        if (!hi_between(V, 1e-27, 1e6)) return false;
+        const double z = V * qn;
+        if (!((unsigned)(__double2hiint(z) & 0x7fffffff) < (unsigned)__double2hiint(600.0))) return false;
+        const double ic = p.Dc * fm_rcp(V);
+        Th = fma(p.ThetaOld - ic, fm_exp(z), ic);
+        if (!hi_between(Th, 1e-30, 1e30)) return false;
+        lv = fm_log(V * 1e9);   // V / V0
+        lt = fm_log(Th * kth);
+        W = fma(Baa, lv, fma(Bab, lt, fma(-Be, V, A0)));
+        return true;
+    };
+    const double DV = p.VOld * 0.01;
+    double V = p.VOld * 1e-10, Th, lv, lt, W, Th2, l2, t2, W2;
+    if (!eval(V, Th, lv, lt, W)) return false;
+    int it = 0;
+    for (;;) {
+        ++it;
+        const double VTest = V, f = V - W;
+        if (!eval(V + DV, Th2, l2, t2, W2)) return false;
+        const double fu = (V + DV) - W2;
+        V = VTest - f * DV * fm_rcp(fu - f);
+        if (!hi_between(V, 1e-27, 1e6) || !eval(V, Th, lv, lt, W)) return false;
+        if (!(fabs(VTest - V) > kConv * V)) break;
+        if (it >= 98) return false;
+    }
+    o.V = V;
+    o.Friction = p.Friction0 + p.a * lv + p.b * lt;
+    o.Disp = p.DispOld + (p.VOld + V) * 0.5 * Dt;
+    o.Theta = Th;
+    o.Dt = Dt; o.Instab = 0; o.Flag = 1; o.Iterations = it;
+    return true;
+}
+
 // The reference loops, one lane or a lane pair per patch, for what
-// solve_lowv_newton leaves.  Inlined: a call from the persistent kernel makes
+// the two solvers above leave.  Inlined: a call from the persistent kernel makes
 // the operator warps save their sums around it (12,813 patches x 4: 3.3 times
 // slower).  `in` is a copy, so that the caller's operands stay in registers.
 static __device__ __forceinline__ PatchOut solve_reference(PatchIn in, bool high, bool pair, double Dt, double eta,
@@ -580,17 +652,22 @@ static __device__ __forceinline__ PatchOut solve_reference(PatchIn in, bool high
                 : solve_lowv(in, Dt, eta, alpha, dr, SwitchV, err);
 }
 
-// InterpolateFromStressChange for one patch column.
-__device__ __forceinline__ void interp_ext(int64_t nt, const double* __restrict__ t,
-                                           const double* __restrict__ en,
-                                           const double* __restrict__ es,
-                                           const double* __restrict__ ep, int64_t N, int64_t i,
-                                           double Time, double& dn, double& ds, double& dp) {
-    int64_t idx = 0;
+// InterpolateFromStressChange: the sample segment that Time falls into (0 before
+// the first sample, nt from the last on) and the fraction of it, then a patch's
+// values there.
+__device__ __forceinline__ void ext_segment(int64_t nt, const double* __restrict__ t, double Time, int& idx,
+                                            double& f) {
+    idx = 0;
+    f = 0.0;
     for (int64_t k = 1; k <= nt; ++k)
-        if (Time >= t[k - 1]) idx = k;
+        if (Time >= t[k - 1]) idx = (int)k;
+    if (idx == 0) f = Time / t[0];
+    else if (idx < nt) f = (Time - t[idx - 1]) / (t[idx] - t[idx - 1]);
+}
+__device__ __forceinline__ void interp_ext_at(int idx, double f, int64_t nt, const double* __restrict__ en,
+                                              const double* __restrict__ es, const double* __restrict__ ep, int64_t N,
+                                              int64_t i, double& dn, double& ds, double& dp) {
     if (idx == 0) {
-        const double f = Time / t[0];
         dn = f * (en[i] - 0.0) + 0.0;
         ds = f * (es[i] - 0.0) + 0.0;
         dp = f * (ep[i] - 0.0) + 0.0;
@@ -599,12 +676,19 @@ __device__ __forceinline__ void interp_ext(int64_t nt, const double* __restrict_
         ds = es[(nt - 1) * N + i];
         dp = ep[(nt - 1) * N + i];
     } else {
-        const double f = (Time - t[idx - 1]) / (t[idx] - t[idx - 1]);
-        const int64_t lo = (idx - 1) * N + i, hi = idx * N + i;
+        const int64_t lo = (int64_t)(idx - 1) * N + i, hi = (int64_t)idx * N + i;
         dn = f * (en[hi] - en[lo]) + en[lo];
         ds = f * (es[hi] - es[lo]) + es[lo];
         dp = f * (ep[hi] - ep[lo]) + ep[lo];
     }
+}
+__device__ __forceinline__ void interp_ext(int64_t nt, const double* __restrict__ t, const double* __restrict__ en,
+                                           const double* __restrict__ es, const double* __restrict__ ep, int64_t N,
+                                           int64_t i, double Time, double& dn, double& ds, double& dp) {
+    int idx;
+    double f;
+    ext_segment(nt, t, Time, idx, f);
+    interp_ext_at(idx, f, nt, en, es, ep, N, i, dn, ds, dp);
 }
 
 }  // namespace sim

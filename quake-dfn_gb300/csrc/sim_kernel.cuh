@@ -69,6 +69,7 @@ struct SimParams {
     int nblk;                        // thread blocks that run this context (its grid barrier's size)
     int evolution_dr, interp_at_told, hmat;
     double eta, sigma_min, switch_v, dt_cut, rupture_dt, max_dt, alpha_evo;
+    double r_dt_cut;                 // 1/dt_cut, correctly rounded
     int64_t record_step, max_records;
     // per [R][N] constants
     const double *a, *b, *Dc, *F0, *tau0, *sigma0, *Vconst, *mass, *omega;
@@ -151,34 +152,55 @@ struct SimParams {
 
 namespace {
 
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* ptr) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
+    return v;
+}
+
+// One block's arrival and wait at the grid barrier of p's blocks (one thread of
+// the block; the block's threads meet before and after).  The arrival's
+// acq_rel addition publishes what the block wrote -- it has met at a block
+// barrier -- and the acquiring reads of the generation take in what the others
+// published, so no full memory fences are needed.  While it waits a thread
+// reads the generation alone, and the clock and the error flag every 16th time:
+// each is a round trip to L2, and the wait's period is part of every step's
+// latency.  `close`: a counter that the last block to arrive closes before it
+// releases the others.  Returns false when the deadline has passed or a block
+// has raised the error flag.
+// Against full fences, both reads in every round and a sleep after each, with the
+// block rule in configure_launch changed along with it: 800 patches, FP64, 200
+// steps through `main` 11.8 -> 9.6 ms; 49 patches, 32 steps 873 -> 775 us.
+__device__ bool barrier_arrive_wait(const SimParams& p, uint64_t deadline_ns, unsigned long long* close) {
+    const unsigned my_gen = ld_acquire_u32(p.bar_gen);
+    unsigned prev;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(p.bar_count) : "memory");
+    if (prev == (unsigned)p.nblk - 1) {
+        if (close) atomicOr(close, 1ull << 62);   // kSpecClosed
+        atomicExch(p.bar_count, 0u);
+        asm volatile("red.add.release.gpu.global.u32 [%0], 1;" ::"l"(p.bar_gen) : "memory");
+        return true;
+    }
+    for (unsigned k = 1; ld_acquire_u32(p.bar_gen) == my_gen; ++k) {
+        if (k % 16 == 0) {
+            if (globaltimer_ns() > deadline_ns + 2000000000ull || *(volatile int*)p.gerr != 0) {
+                atomicExch(p.gerr, QDFN_ERR_TIMEOUT);
+                return false;
+            }
+            __nanosleep(32);
+        }
+    }
+    return true;
+}
+
 // bounded grid barrier; returns false on timeout, or as soon as another block
-// has raised the error flag (all CTAs then return)
+// has raised the error flag (all CTAs then return).  A context of one block
+// only meets its own threads.
 __device__ bool grid_barrier(const SimParams& p, uint64_t deadline_ns) {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned* gen = p.bar_gen;
-        const unsigned my_gen = *gen;
-        __threadfence();
-        const unsigned prev = atomicAdd(p.bar_count, 1u);
-        int ok = 1;
-        if (prev == (unsigned)p.nblk - 1) {
-            atomicExch(p.bar_count, 0u);
-            __threadfence();
-            atomicAdd((unsigned*)p.bar_gen, 1u);
-        } else {
-            while (*gen == my_gen) {
-                if (globaltimer_ns() > deadline_ns + 2000000000ull || *(volatile int*)p.gerr != 0) {
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        if (!ok) atomicExch(p.gerr, QDFN_ERR_TIMEOUT);
-        s_ok = ok;
-    }
+    if (p.nblk == 1) return true;
+    if (threadIdx.x == 0) s_ok = barrier_arrive_wait(p, deadline_ns, nullptr) ? 1 : 0;
     __syncthreads();
     return s_ok != 0;
 }
@@ -201,6 +223,17 @@ __device__ __forceinline__ unsigned long long key_op(int op, unsigned long long 
     return op == 0 ? (a > b ? a : b) : (a < b ? a : b);
 }
 
+// Reduction of the keys of the warp's lanes `m`: the upper halves, then the lower
+// ones among those that hold it (two integer warp reductions, where a 64-bit
+// shuffle tree takes five rounds of two shuffles and a select)
+__device__ __forceinline__ unsigned long long warp_key(int op, unsigned m, unsigned long long key) {
+    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+    const unsigned h = op == 0 ? __reduce_max_sync(m, hi) : __reduce_min_sync(m, hi);
+    const unsigned l = op == 0 ? __reduce_max_sync(m, hi == h ? lo : 0u)
+                               : __reduce_min_sync(m, hi == h ? lo : 0xffffffffu);
+    return ((unsigned long long)h << 32) | l;
+}
+
 // block-wide reduction of R*K doubles with op (0 = max, 1 = min)
 template <int K>
 __device__ void block_reduce(double (&v)[kMaxInst][K], const int (&ops)[K], int R) {
@@ -209,9 +242,7 @@ __device__ void block_reduce(double (&v)[kMaxInst][K], const int (&ops)[K], int 
     for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            unsigned long long x = ord_key(v[r][k]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x = key_op(ops[k], x, __shfl_xor_sync(0xffffffffu, x, o));
+            const unsigned long long x = warp_key(ops[k], 0xffffffffu, ord_key(v[r][k]));
             if (lane == 0) s_buf[wid][r][k] = x;
         }
     __syncthreads();
@@ -233,7 +264,7 @@ __device__ void block_reduce(double (&v)[kMaxInst][K], const int (&ops)[K], int 
 
 // Reduce K fields of every CTA's partial for instance r (slot layout of
 // SimParams::red) across the grid: one warp, lanes stride over the CTAs, then
-// a shuffle tree.  Every lane returns the result.  min/max only: exact, so the
+// a warp reduction.  Every lane returns the result.  min/max only: exact, so the
 // result does not depend on the order.
 template <int K>
 __device__ __forceinline__ void grid_fields(const double* slots_base, int nblk, int R, int r,
@@ -250,9 +281,7 @@ __device__ __forceinline__ void grid_fields(const double* slots_base, int nblk, 
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[k] = key_op(ops[k], acc[k], __shfl_xor_sync(0xffffffffu, acc[k], o));
-        out[k] = ord_val(acc[k]);
+        out[k] = ord_val(warp_key(ops[k], 0xffffffffu, acc[k]));
     }
 }
 
@@ -300,30 +329,7 @@ constexpr unsigned long long kSpecClosed = 1ull << 62;
 __device__ bool grid_barrier_solvers(const SimParams& p, uint64_t deadline_ns, unsigned long long* close) {
     __shared__ int s_ok;
     solver_sync();
-    if (threadIdx.x == kOpThreads) {
-        volatile unsigned* gen = p.bar_gen;
-        const unsigned my_gen = *gen;
-        __threadfence();
-        const unsigned prev = atomicAdd(p.bar_count, 1u);
-        int ok = 1;
-        if (prev == (unsigned)p.nblk - 1) {
-            atomicOr(close, kSpecClosed);
-            atomicExch(p.bar_count, 0u);
-            __threadfence();
-            atomicAdd((unsigned*)p.bar_gen, 1u);
-        } else {
-            while (*gen == my_gen) {
-                if (globaltimer_ns() > deadline_ns + 2000000000ull || *(volatile int*)p.gerr != 0) {
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        if (!ok) atomicExch(p.gerr, QDFN_ERR_TIMEOUT);
-        s_ok = ok;
-    }
+    if (threadIdx.x == kOpThreads) s_ok = barrier_arrive_wait(p, deadline_ns, close) ? 1 : 0;
     solver_sync();
     return s_ok != 0;
 }
@@ -389,11 +395,6 @@ __device__ __forceinline__ void fence_proxy_async_global() {
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* ptr) {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ptr) : "memory");
-    return v;
-}
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* ptr) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
     return v;
 }
 
@@ -508,11 +509,15 @@ __device__ __forceinline__ void xload(const X* p, X x[R]) {
 // FP64.  FP32/BF16 storage (kPairs): each partial is the tile's (hi, lo) FP32
 // pair; the hi parts are gathered error-free with TwoSum and the lo parts
 // added, all on the FP32 pipe, and the pair becomes a double once per row.
-// Loads are issued in batches (16 chunks per matrix, 8 when one lane sums
-// both; past the last chunk a batch re-reads it and skips the sum), so every
+// Loads are issued in batches (16 chunks per matrix, 8 of FP32 pairs when one
+// lane sums both; past the last chunk a batch re-reads it and skips the sum), so every
 // batch costs one memory round trip.
 __device__ __forceinline__ int chunks_of_rb(const SimParams& p, int64_t rb) {
     return rb >= p.rb_small0 ? p.nchunk2 : p.nchunk;
+}
+
+__device__ __forceinline__ int chunks_of_row(const SimParams& p, int64_t i) {
+    return i >= p.rb_small0 * p.ld ? p.nchunk2 : p.nchunk;
 }
 
 // Rows of one solve chunk of the overlapped phase: 16 on lane pairs, 32 with
@@ -568,7 +573,7 @@ template <bool kPairs>
 __device__ __forceinline__ double sum_partials_side(const SimParams& p, int r, int64_t i, int side, int ppar) {
     const int64_t cs = (int64_t)p.R * p.N;
     const int64_t base = (int64_t)ppar * p.part_stride + (int64_t)r * p.N + i;
-    const int nch = chunks_of_rb(p, i / p.ld);
+    const int nch = chunks_of_row(p, i);
     const double* part = side == 0 ? p.part_s : p.part_n;
     if constexpr (kPairs) {
         const float2* ps = reinterpret_cast<const float2*>(part) + base;
@@ -602,7 +607,7 @@ __device__ __forceinline__ void sum_partials(const SimParams& p, int r, int64_t 
                                              int ppar = 0) {
     const int64_t cs = (int64_t)p.R * p.N;
     const int64_t base = (int64_t)ppar * p.part_stride + (int64_t)r * p.N + i;
-    const int nch = chunks_of_rb(p, i / p.ld);
+    const int nch = chunks_of_row(p, i);
     if constexpr (kPairs) {
         const float2* ps = reinterpret_cast<const float2*>(p.part_s) + base;
         const float2* pn = reinterpret_cast<const float2*>(p.part_n) + base;
@@ -628,16 +633,16 @@ __device__ __forceinline__ void sum_partials(const SimParams& p, int r, int64_t 
         const double* ps = p.part_s + base;
         const double* pn = p.part_n + base;
         double as = 0, an = 0;
-        for (int c = 0; c < nch; c += 8) {
-            double ts[8], tn[8];
+        for (int c = 0; c < nch; c += 16) {
+            double ts[16], tn[16];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < 16; ++k) {
                 const int cc = min(c + k, nch - 1);   // (past the end: a repeat, not summed)
                 ts[k] = __ldcg(ps + cc * cs);
                 tn[k] = __ldcg(pn + cc * cs);
             }
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
+            for (int k = 0; k < 16; ++k)
                 if (c + k < nch) { as += ts[k]; an += tn[k]; }
         }
         ss = as;
@@ -1024,14 +1029,14 @@ __device__ __forceinline__ double next_dt(const SimParams& p, double vmax, doubl
                                           double dt_prev, bool* empty) {
     *empty = (any == 0);
     if (vnan != 0) vmax = NAN;
-    dtmin = dtmin / p.dt_cut;
+    dtmin = sim::div_by(dtmin, sim::recip_pre(p.dt_cut, p.r_dt_cut));   // dtmin / dt_cut
     double DtRef;
     if (vmax > p.switch_v) DtRef = p.rupture_dt;
     else if (dtmin > p.max_dt) DtRef = p.max_dt;
     else DtRef = dtmin;
     double Dt = dt_prev;
     if (DtRef <= p.rupture_dt) Dt = DtRef;
-    else if (Dt < DtRef / 1.2) Dt = Dt * 1.2;
+    else if (Dt < sim::div_by(DtRef, sim::Recip{1.2, 1.0 / 1.2, true})) Dt = Dt * 1.2;
     else Dt = DtRef;
     return Dt;
 }
@@ -1066,6 +1071,17 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
     // host keeps, and the next launch's controller starts from)
     __shared__ double s_T[kMaxInst], s_dt[kMaxInst], s_dtn[kMaxInst], s_dta[kMaxInst];
     __shared__ double s_rdt[kMaxInst];   // 1/s_dt, correctly rounded, formed before each solve pass
+    // where the external stress of a solve pass lies in its samples: segment and
+    // fraction, the same for every patch, formed with s_rdt
+    __shared__ int s_ext_i[kMaxInst];
+    __shared__ double s_ext_f[kMaxInst];
+    auto pass_scalars = [&](int r) {
+        s_rdt[r] = 1.0 / s_dt[r];
+        if (p.n_ext > 0) {
+            const double tq = p.interp_at_told ? s_T[r] : s_T[r] + s_dt[r];
+            sim::ext_segment(p.n_ext, p.ext_t, tq, s_ext_i[r], s_ext_f[r]);
+        }
+    };
     __shared__ int64_t s_step[kMaxInst], s_nrec[kMaxInst];
     __shared__ int s_done[kMaxInst], s_fail[kMaxInst], s_stop, s_par;
     __shared__ int s_fill_stop, s_fill_counted;   // fill mode: every member has its nsteps; this one counted
@@ -1122,6 +1138,22 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
     };
     auto red_min = [&](int r, int k, double x) { atomicMin(&s_red[r][k], ord_key(x)); };
     auto red_max = [&](int r, int k, double x) { atomicMax(&s_red[r][k], ord_key(x)); };
+    // the same for what every lane contributes: the lanes of the calling warp
+    // that are here together and work on the same instance reduce first, and one
+    // of them does the atomic (64-bit shared atomics on one word go lane by lane)
+    auto warp_red = [&](bool mx, int r, int k, double x) {
+        unsigned m = __activemask();
+        const int r0 = __shfl_sync(m, r, __ffs(m) - 1);
+        const bool with = r == r0;
+        if (!__all_sync(m, with)) {   // lanes of two instances: each its own atomic
+            if (mx) red_max(r, k, x); else red_min(r, k, x);
+            return;
+        }
+        const unsigned long long t = warp_key(mx ? 0 : 1, m, ord_key(x));
+        if ((threadIdx.x & 31) == __ffs(m) - 1) {
+            if (mx) atomicMax(&s_red[r][k], t); else atomicMin(&s_red[r][k], t);
+        }
+    };
 
     // ------------------------------------------------------------ prologue
     // time control of the first step from the state as it stands (later steps
@@ -1217,7 +1249,7 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
         const bool use_order = !HM && sizeof(X) == 4 && p.rb_ordered && p.n_rb <= kMaxOrder;
         const bool pre = it > 0 && s_next_valid == it;
         if (use_order && !pre && threadIdx.x < 32) rb_order(p, cpar, s_order[it & 1]);
-        if (threadIdx.x >= 32 && threadIdx.x < 32 + R) s_rdt[threadIdx.x - 32] = 1.0 / s_dt[threadIdx.x - 32];
+        if (threadIdx.x >= 32 && threadIdx.x < 32 + R) pass_scalars(threadIdx.x - 32);
         red_init();
         __syncthreads();
         const X* xdc = reinterpret_cast<const X*>(p.xd) + (size_t)par * p.xd_stride;
@@ -1262,10 +1294,8 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                     }
                     tld_q = -ss;   // ELSM * (0 - DispOld)
                     knd_q = sn;    // StiffnessMatrixNormal * DispOld
-                    if (writer) {
-                        p.tld[q] = tld_q;
-                        p.knd[q] = knd_q;
-                    }
+                    // (stored with the results, so that the loads of the patch's
+                    // state do not wait behind the stores)
                 }
             } else {
                 tld_q = p.tld[q];
@@ -1273,10 +1303,8 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
             }
             const double Dt = s_dt[r];
             double dsn = 0, dss = 0, dsp = 0;
-            if (p.n_ext > 0) {
-                const double tq = p.interp_at_told ? s_T[r] : s_T[r] + Dt;
-                sim::interp_ext(p.n_ext, p.ext_t, p.ext_n, p.ext_s, p.ext_p, N, i, tq, dsn, dss, dsp);
-            }
+            if (p.n_ext > 0)
+                sim::interp_ext_at(s_ext_i[r], s_ext_f[r], p.n_ext, p.ext_n, p.ext_s, p.ext_p, N, i, dsn, dss, dsp);
             double sig = knd_q + p.sigma0[q] + dsn;
             if (sig < p.sigma_min) sig = p.sigma_min;
             const double VOld = QDFN_CUR(V, Vn)[q];
@@ -1293,9 +1321,11 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                 int err = 0;
                 sim::PatchOut o;
                 const int swq = QDFN_CUR(sw, sw_n)[q];
-                if (swq == 1 || !sim::solve_lowv_newton(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, o))
+                if (!(swq == 1 ? sim::solve_highv_usual(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, o)
+                               : sim::solve_lowv_newton(pin, Dt, p.eta, p.alpha_evo, p.evolution_dr, o)))
                     o = sim::solve_reference(pin, swq == 1, pair, Dt, p.eta, p.alpha_evo, p.evolution_dr, p.switch_v, err);
                 if (!writer) return;
+                if (!HM && first) { p.tld[q] = tld_q; p.knd[q] = knd_q; }
                 if (p.sw_used) p.sw_used[q] = (unsigned char)swq;
                 QDFN_NXT(V, Vn)[q] = o.V; QDFN_NXT(fric, fn)[q] = o.Friction; QDFN_NXT(D, Dn)[q] = o.Disp;
                 QDFN_NXT(theta, thn)[q] = o.Theta; QDFN_NXT(sig_old, sn)[q] = sig;
@@ -1304,7 +1334,7 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                 else { ++n_lo; it_lo += o.Iterations; }
                 if (err) red_min(r, 3, (double)err);
                 if (o.Flag != 1) red_min(r, 0, (double)o.Flag);
-                red_min(r, 1, o.Dt);
+                warp_red(false, r, 1, o.Dt);
                 if (o.Instab == 4) red_max(r, 2, 1.0);
                 if (o.Flag == 0) {   // Main_D :242-249, applied by the patch's owner
                     if (o.Instab == 3) QDFN_CUR(sw, sw_n)[q] = 1;
@@ -1317,6 +1347,7 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                 }
             } else {
                 if (!writer) return;   // loading faults (Solvers :370-377)
+                if (!HM && first) { p.tld[q] = tld_q; p.knd[q] = knd_q; }
                 if (p.sw_used) p.sw_used[q] = 2;
                 const double Vc = p.Vconst[q];
                 const double Dn = QDFN_CUR(D, Dn)[q] + Vc * Dt;
@@ -1324,7 +1355,7 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                 QDFN_NXT(theta, thn)[q] = QDFN_CUR(theta, thn)[q]; QDFN_NXT(sig_old, sn)[q] = 1e10;
                 p.dtall[q] = Dt;
                 p.instab[q] = 0; p.flag[q] = 1;
-                red_min(r, 1, Dt);
+                warp_red(false, r, 1, Dt);
                 Vnew = Vc;
                 if constexpr (!HM) {
                     const double d0 = offs ? QDFN_CUR(D, Dn)[(int64_t)r * N] : 0.0;
@@ -1343,9 +1374,23 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
             }
             if (p.has_unstable[r] ? (p.unstable[q] != 0) : (i < Ns)) {
                 if (isnan(Vnew)) red_max(r, 5, 1.0);
-                else red_max(r, 4, Vnew);
-                const double qa = fabs(Vnew / A);
-                if (!isnan(qa) && qa != 0) { red_max(r, 7, 1.0); red_min(r, 6, qa); }
+                else warp_red(true, r, 4, Vnew);
+                // only the smallest |V/A| matters: formed where it can be below
+                // the block's so far, by an FP32 estimate where that has the range
+                const float vf = sim::to_float(fabs(Vnew)), af = sim::to_float(fabs(A));
+                const bool ranged = sim::hi_between(fabs(Vnew), 1e-30, 1e30) && sim::hi_between(fabs(A), 1e-30, 1e30);
+                const float est = __fdividef(vf, af);
+                const double seen = ord_val(*(volatile unsigned long long*)&s_red[r][6]);
+                if (ranged && est > 1e-18f && est < 1e18f && sim::hi_between(seen, 1e-20, 1e18) &&
+                    est > 1.00001f * sim::to_float(seen)) {
+                    if (s_red[r][7] != ord_key(1.0)) s_red[r][7] = ord_key(1.0);   // (every writer stores 1)
+                } else {
+                    const double qa = fabs(Vnew / A);
+                    if (!isnan(qa) && qa != 0) {
+                        if (s_red[r][7] != ord_key(1.0)) s_red[r][7] = ord_key(1.0);
+                        warp_red(false, r, 6, qa);
+                    }
+                }
             }
         };
 #undef QDFN_CUR
@@ -1614,7 +1659,7 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
             if (HM || sizeof(X) == 8 || !first) {   // FP32/BF16 dense pass 0 ran alongside the operator
                 if (!first) {
                     red_init();
-                    if (threadIdx.x < R) s_rdt[threadIdx.x] = 1.0 / s_dt[threadIdx.x];
+                    if (threadIdx.x < R) pass_scalars(threadIdx.x);
                     __syncthreads();
                 }
                 // every CTA takes an equal contiguous range of (instance, patch)
@@ -1631,7 +1676,9 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                     }
                 }
                 for (int64_t q = (int64_t)blk * per_cta + threadIdx.x; q < q_end; q += kSimThreads) {
-                    const int r = (int)(q / N);
+                    int r = 0;   // q / N, q < R N
+#pragma unroll
+                    for (int k = 1; k < R; ++k) r += q >= k * N ? 1 : 0;
                     if (s_done[r]) continue;
                     solve_item(q, r, q - (int64_t)r * N, prod_here, false);
                 }
