@@ -1,5 +1,5 @@
 // Kernels of the discrete adjoint of the stepped system (qdfn_adjoint_run in
-// sim.cu drives them, one reverse step at a time):
+// sim.cu queues them, one reverse step after another):
 //
 //   k_adj_local      per (instance, patch): the vector-Jacobian product of the
 //                    patch's converged step (adjoint.cuh) -- adjoints of the
@@ -14,9 +14,9 @@
 //                    storage in FP64; one partial per (row block, instance,
 //                    column), summed in row-block order by k_adj_combine
 //   k_adj_combine    lambda_D(old) = local part - E^T lambda_TLD + Kn^T lambda_sigma
-//   k_adj_dtctl      the time-step controller's reductions of a state (max V,
-//                    min |V/Accel| and its patch), to route the adjoint of dt
-//                    through the patch that set it
+//   k_adj_control    the adjoint of dt, routed through the controller's choice of
+//                    it (through the patch that set min |V/Accel|, or the step
+//                    before), and the seeds of the state
 // The transposed product is the reverse pass's HBM-bound kernel (the operator
 // bytes once per product); the local products are FP64 (dual numbers).
 #include <cuda_bf16.h>
@@ -32,7 +32,7 @@ namespace qdfn {
 namespace {
 
 constexpr int kAdjThreads = 256;
-
+constexpr int kLocalThreads = 64;   // k_adj_local: a long chain per patch, so small blocks on many SMs
 // slope d/dt of the piecewise-linear external stress of patch column i at time
 // Time (InterpolateFromStressChange, Functions_Solvers.jl:465-540): the ramp
 // from zero before the first sample, the segment's slope inside, zero after the
@@ -54,8 +54,14 @@ __device__ inline void interp_slope(int64_t nt, const double* t, const double* e
     }
 }
 
-__global__ void __launch_bounds__(kAdjThreads) k_adj_local(AdjLocalArgs a) {
-    __shared__ double s_dt[kAdjMaxInst][kAdjThreads / 32], s_tx[kAdjMaxInst][kAdjThreads / 32];
+// by dual numbers: high-velocity solves and the slip law.  Out of line: its 11
+// directions fill the registers
+__device__ __noinline__ bool dual_vjp(const adj::PatchX& x, double lV, double lD, double lth, double lA, double* o) {
+    return adj::local_vjp(x, lV, lD, lth, lA, o);
+}
+
+__global__ void __launch_bounds__(kLocalThreads) k_adj_local(AdjLocalArgs a) {
+    __shared__ double s_dt[kAdjMaxInst][kLocalThreads / 32], s_tx[kAdjMaxInst][kLocalThreads / 32];
     const int64_t RN = (int64_t)a.R * a.N;
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     double ldt = 0, ltx = 0;   // this thread's share of d/d(dt) and of d/d(external-stress time)
@@ -90,7 +96,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_local(AdjLocalArgs a) {
             }
             x.dtau = dtau;
             double o[adj::kDirs - 1];
-            if (adj::local_vjp(x, lV, lD, lth, lA, o)) {
+            if (!x.high && x.dr == 1 ? adj::local_vjp_low(x, lV, lD, lth, lA, o) : dual_vjp(x, lV, lD, lth, lA, o)) {
                 lDloc = o[adj::dDold - 1];
                 lVold = o[adj::dVold - 1];
                 lThold = o[adj::dThold - 1];
@@ -125,21 +131,10 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_local(AdjLocalArgs a) {
     __syncthreads();
     if (threadIdx.x < a.R) {
         double u = 0, v = 0;
-        for (int w = 0; w < kAdjThreads / 32; ++w) { u += s_dt[threadIdx.x][w]; v += s_tx[threadIdx.x][w]; }
+        for (int w = 0; w < kLocalThreads / 32; ++w) { u += s_dt[threadIdx.x][w]; v += s_tx[threadIdx.x][w]; }
         a.blk_dt[(int64_t)blockIdx.x * a.R + threadIdx.x] = u;
         a.blk_tx[(int64_t)blockIdx.x * a.R + threadIdx.x] = v;
     }
-}
-
-// sums of the per-block partials, in block order: out[r] = dt adjoint, out[R + r] = time adjoint
-__global__ void k_adj_sum_blocks(int nblk, int R, const double* __restrict__ bdt, const double* __restrict__ btx,
-                                 double* __restrict__ out) {
-    const int r = threadIdx.x;
-    if (r >= R) return;
-    double u = 0, v = 0;
-    for (int b = 0; b < nblk; ++b) { u += bdt[(int64_t)b * R + r]; v += btx[(int64_t)b * R + r]; }
-    out[r] = u;
-    out[R + r] = v;
 }
 
 // ---------------------------------------------------------------------------
@@ -163,37 +158,55 @@ __device__ __forceinline__ void two_sum(float& hi, float& lo, float p) {
     hi = s;
 }
 
-// one warp per (row block, column): partial[rb][side][r][j]
+// One warp per (row block, column): partial[rb][side][r][j].  The column's entries
+// of both matrices are loaded before any is used (2 x 16 loads of a lane in
+// flight: the products are bound by HBM or L2 latency), and the warp's x values
+// stay in registers over its columns where they fit (one instance).
 template <class F, int R>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_transpose_f32(AdjTransArgs a) {
     extern __shared__ float xs[];   // [2 sides][R][rpb]
+    constexpr int rpb = 512, kM = rpb / 32;   // the forward's row block in 4-byte formats
     const int rb = blockIdx.y;
-    const int64_t rpb = a.rpb, N = a.N;
-    for (int64_t k = threadIdx.x; k < 2 * R * rpb; k += blockDim.x) {
-        const int side = (int)(k / (R * rpb));
-        const int r = (int)((k / rpb) % R);
-        const int64_t i = rb * rpb + k % rpb;
+    const int64_t N = a.N;
+    for (int k = threadIdx.x; k < 2 * R * rpb; k += blockDim.x) {
+        const int side = k / (R * rpb);
+        const int r = (k / rpb) % R;
+        const int64_t i = (int64_t)rb * rpb + k % rpb;
         const double* src = side == 0 ? a.x_s : a.x_n;
         xs[k] = i < N ? (float)src[(int64_t)r * N + i] : 0.f;
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
+    float xr[2][R == 1 ? kM : 1];
+    if constexpr (R == 1) {
+#pragma unroll
+        for (int side = 0; side < 2; ++side)
+#pragma unroll
+            for (int m = 0; m < kM; ++m) xr[side][m] = xs[side * rpb + lane + 32 * m];
+    }
     for (int64_t j = (int64_t)blockIdx.x * nw + wid; j < N; j += (int64_t)gridDim.x * nw) {
-        const int64_t base = ((int64_t)rb * N + j) * rpb;
+        const int64_t base = ((int64_t)rb * N + j) * rpb + lane;
+        float e[2][kM];
+#pragma unroll
+        for (int m = 0; m < kM; ++m) e[0][m] = F::get(a.E, base + 32 * m);
+#pragma unroll
+        for (int m = 0; m < kM; ++m) e[1][m] = F::get(a.Kn, base + 32 * m);
+#pragma unroll
         for (int side = 0; side < 2; ++side) {
-            const void* M = side == 0 ? a.E : a.Kn;
             float hi[R], lo[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) { hi[r] = 0.f; lo[r] = 0.f; }
-            for (int64_t k = lane; k < rpb; k += 32) {
-                const float m = F::get(M, base + k);
 #pragma unroll
-                for (int r = 0; r < R; ++r) hi[r] = fmaf(m, xs[(side * R + r) * rpb + k], hi[r]);
-            }
+            for (int m = 0; m < kM; ++m)
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    hi[r] = fmaf(e[side][m], R == 1 ? xr[side][R == 1 ? m : 0] : xs[(side * R + r) * rpb + lane + 32 * m],
+                                 hi[r]);
             // warp tree in error-free pairs
 #pragma unroll
             for (int r = 0; r < R; ++r)
+#pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     const float h2 = __shfl_xor_sync(0xffffffffu, hi[r], o);
                     const float l2 = __shfl_xor_sync(0xffffffffu, lo[r], o);
@@ -211,12 +224,13 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_transpose_f32(AdjTransArgs 
 template <int R>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_transpose_f64(AdjTransArgs a) {
     extern __shared__ double xd[];   // [2 sides][R][rpb]
+    constexpr int rpb = 256, kM = rpb / 32;
     const int rb = blockIdx.y;
-    const int64_t rpb = a.rpb, N = a.N;
-    for (int64_t k = threadIdx.x; k < 2 * R * rpb; k += blockDim.x) {
-        const int side = (int)(k / (R * rpb));
-        const int r = (int)((k / rpb) % R);
-        const int64_t i = rb * rpb + k % rpb;
+    const int64_t N = a.N;
+    for (int k = threadIdx.x; k < 2 * R * rpb; k += blockDim.x) {
+        const int side = k / (R * rpb);
+        const int r = (k / rpb) % R;
+        const int64_t i = (int64_t)rb * rpb + k % rpb;
         const double* src = side == 0 ? a.x_s : a.x_n;
         xd[k] = i < N ? src[(int64_t)r * N + i] : 0.0;
     }
@@ -224,19 +238,24 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_transpose_f64(AdjTransArgs 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nw = blockDim.x >> 5;
     for (int64_t j = (int64_t)blockIdx.x * nw + wid; j < N; j += (int64_t)gridDim.x * nw) {
-        const int64_t base = ((int64_t)rb * N + j) * rpb;
+        const int64_t base = ((int64_t)rb * N + j) * rpb + lane;
+        double e[2][kM];
+#pragma unroll
+        for (int m = 0; m < kM; ++m) e[0][m] = reinterpret_cast<const double*>(a.E)[base + 32 * m];
+#pragma unroll
+        for (int m = 0; m < kM; ++m) e[1][m] = reinterpret_cast<const double*>(a.Kn)[base + 32 * m];
+#pragma unroll
         for (int side = 0; side < 2; ++side) {
-            const double* M = reinterpret_cast<const double*>(side == 0 ? a.E : a.Kn);
             double acc[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) acc[r] = 0.0;
-            for (int64_t k = lane; k < rpb; k += 32) {
-                const double m = M[base + k];
 #pragma unroll
-                for (int r = 0; r < R; ++r) acc[r] = fma(m, xd[(side * R + r) * rpb + k], acc[r]);
-            }
+            for (int m = 0; m < kM; ++m)
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[r] = fma(e[side][m], xd[(side * R + r) * rpb + lane + 32 * m], acc[r]);
 #pragma unroll
             for (int r = 0; r < R; ++r)
+#pragma unroll
                 for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
             if (lane == 0)
 #pragma unroll
@@ -247,7 +266,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_transpose_f64(AdjTransArgs 
 
 // lambda_D_old = local part - sum_rb E^T partials + sum_rb Kn^T partials (row-block order)
 __global__ void k_adj_combine(int64_t N, int R, int64_t nrb, const double* __restrict__ part,
-                              const double* __restrict__ dloc, double* __restrict__ out) {
+                              const double* __restrict__ dloc, double* __restrict__ out,
+                              double* __restrict__ zero) {
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= (int64_t)R * N) return;
     const int r = (int)(q / N);
@@ -258,48 +278,88 @@ __global__ void k_adj_combine(int64_t N, int R, int64_t nrb, const double* __res
         sk += part[((rb * 2 + 1) * R + r) * N + j];
     }
     out[q] = dloc[q] - se + sk;
+    zero[q] = 0.0;
 }
 
-// the controller's reductions of a state, one block per instance: out[r*5 ..]
-// = {max V, V is NaN, min |V/A| (NaN and 0 left out), any usable, its patch}
-__global__ void __launch_bounds__(kAdjThreads) k_adj_dtctl(int64_t N, int64_t Ns, const double* __restrict__ V,
-                                                           const double* __restrict__ A,
-                                                           const unsigned char* __restrict__ unstable,
-                                                           const int* __restrict__ has_unstable,
-                                                           double* __restrict__ out) {
+// One block per instance: the controller's reductions of the state that the
+// step's Dt was chosen from (max V, min |V/A| and its patch, NaN and 0 left out),
+// the sums of adj_local's block partials in block order, and then, by one
+// thread, where the adjoint of Dt goes and the state's seeds in their order.
+constexpr int kCtlThreads = 512;
+__global__ void __launch_bounds__(kCtlThreads) k_adj_control(AdjControlArgs a) {
     const int r = blockIdx.x;
-    __shared__ double s_vmax[kAdjThreads], s_q[kAdjThreads];
-    __shared__ long long s_k[kAdjThreads];
-    __shared__ int s_nan[kAdjThreads];
+    __shared__ double s_vmax[kCtlThreads / 32], s_q[kCtlThreads / 32];
+    __shared__ long long s_k[kCtlThreads / 32];
+    __shared__ int s_nan;
     double vmax = -INFINITY, qmin = INFINITY;
     long long kmin = -1;
-    int vnan = 0;
-    for (int64_t i = threadIdx.x; i < N; i += blockDim.x) {
-        const int64_t q = (int64_t)r * N + i;
-        const bool ctl = has_unstable[r] ? (unstable[q] != 0) : (i < Ns);
-        if (!ctl) continue;
-        const double v = V[q];
-        if (isnan(v)) vnan = 1;
-        else vmax = fmax(vmax, v);
-        const double qa = fabs(v / A[q]);
-        if (!isnan(qa) && qa != 0 && qa < qmin) { qmin = qa; kmin = i; }
-    }
-    s_vmax[threadIdx.x] = vmax; s_q[threadIdx.x] = qmin; s_k[threadIdx.x] = kmin; s_nan[threadIdx.x] = vnan;
+    if (threadIdx.x == 0) s_nan = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int t = 1; t < blockDim.x; ++t) {
-            vmax = fmax(vmax, s_vmax[t]);
-            vnan |= s_nan[t];
-            if (s_q[t] < qmin || (s_q[t] == qmin && s_k[t] >= 0 && (kmin < 0 || s_k[t] < kmin))) {
-                qmin = s_q[t];
-                kmin = s_k[t];
-            }
+    if (a.V) {
+        const bool has = a.has_unstable[r] != 0;
+        for (int64_t i = threadIdx.x; i < a.N; i += kCtlThreads) {
+            const int64_t q = (int64_t)r * a.N + i;
+            if (!(has ? a.unstable[q] != 0 : i < a.Ns)) continue;
+            const double v = a.V[q];
+            if (isnan(v)) s_nan = 1;   // (every writer stores 1)
+            else vmax = fmax(vmax, v);
+            const double qa = fabs(v / a.A[q]);
+            if (!isnan(qa) && qa != 0 && qa < qmin) { qmin = qa; kmin = i; }
         }
-        out[r * 5 + 0] = vmax;
-        out[r * 5 + 1] = vnan;
-        out[r * 5 + 2] = qmin;
-        out[r * 5 + 3] = kmin >= 0 ? 1.0 : 0.0;
-        out[r * 5 + 4] = (double)kmin;
+        // the smallest |V/A|, of equal ones the first patch
+        auto take = [&](double v, double q, long long k) {
+            vmax = fmax(vmax, v);
+            if (q < qmin || (q == qmin && k >= 0 && (kmin < 0 || k < kmin))) { qmin = q; kmin = k; }
+        };
+        for (int o = 16; o > 0; o >>= 1)
+            take(__shfl_xor_sync(0xffffffffu, vmax, o), __shfl_xor_sync(0xffffffffu, qmin, o),
+                 __shfl_xor_sync(0xffffffffu, kmin, o));
+        if ((threadIdx.x & 31) == 0) {
+            s_vmax[threadIdx.x >> 5] = vmax; s_q[threadIdx.x >> 5] = qmin; s_k[threadIdx.x >> 5] = kmin;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < kCtlThreads / 32; ++w) take(s_vmax[w], s_q[w], s_k[w]);
+    }
+    if (threadIdx.x != 0) return;
+    if (a.V) {
+        double sdt = 0, stx = 0;
+#pragma unroll 8
+        for (int b = 0; b < a.nblk; ++b) { sdt += a.blk_dt[(int64_t)b * a.R + r]; stx += a.blk_tx[(int64_t)b * a.R + r]; }
+        const double ldt = sdt + a.lamT[r] + (a.told ? 0.0 : stx) + a.carry[r];
+        a.lamT[r] += stx;
+        a.carry[r] = 0.0;
+        const double dtn = a.dt_now[r], dtp = a.dt_prev[r];
+        if (s_nan) vmax = NAN;
+        const double dtmin = qmin / a.dt_cut;
+        int src = 0;   // 0 constant, 1 min |V/A| / DtCut, 2 1.2 x previous Dt
+        double ref;
+        if (vmax > a.switch_v) ref = a.rupture_dt;
+        else if (dtmin > a.max_dt) ref = a.max_dt;
+        else { ref = dtmin; src = kmin >= 0 ? 1 : 0; }
+        double dtc;
+        if (ref <= a.rupture_dt) dtc = ref;
+        else if (dtp < ref / 1.2) { dtc = dtp * 1.2; src = 2; }
+        else dtc = ref;
+        const double sc = dtn / dtc;   // the halvings of its retries (1e-3 of an instability: none of these)
+        const double e2 = log2(sc);
+        if (!(sc > 0 && sc <= 1 && fabs(e2 - round(e2)) < 1e-9)) src = 0;
+        if (src == 1) {
+            const int64_t q = (int64_t)r * a.N + kmin;
+            const double Vk = a.V[q], Ak = a.A[q], sg = Vk / Ak < 0 ? -1.0 : 1.0;
+            a.lV[q] += ldt * sc * sg / (Ak * a.dt_cut);
+            a.lA[q] += -ldt * sc * sg * Vk / (Ak * Ak * a.dt_cut);
+        } else if (src == 2) {
+            a.carry[r] = 1.2 * sc * ldt;
+        }
+    }
+    for (int64_t k = a.seed_off[a.state * a.R + r]; k < a.seed_off[a.state * a.R + r + 1]; ++k) {
+        a.lamT[r] += a.seed_val[3 * k + 2];
+        if (a.seed_patch[k] >= 0) {
+            const int64_t q = (int64_t)r * a.N + a.seed_patch[k];
+            a.lV[q] += a.seed_val[3 * k];
+            a.lD[q] += a.seed_val[3 * k + 1];
+        }
     }
 }
 
@@ -318,41 +378,19 @@ void launch_transpose_R(int prec, const AdjTransArgs& a, cudaStream_t st) {
     }
 }
 
-// sparse additions to the adjoint state: lV[idx[k]] += v[k], lD[idx[k]] += v[n+k], lA[idx[k]] += v[2n+k]
-// (one thread, in order, so repeated indices add up deterministically)
-__global__ void k_adj_add(int n, const int64_t* __restrict__ idx, const double* __restrict__ v, double* lV,
-                          double* lD, double* lA) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (int k = 0; k < n; ++k) {
-        const int64_t q = idx[k];
-        lV[q] += v[k];
-        lD[q] += v[n + k];
-        lA[q] += v[2 * n + k];
-    }
-}
-
 }  // namespace
 
-int adj_add(int n, const int64_t* idx, const double* vals, double* lV, double* lD, double* lA, cudaStream_t st) {
-    if (n <= 0) return QDFN_OK;
-    k_adj_add<<<1, 1, 0, st>>>(n, idx, vals, lV, lD, lA);
-    QDFN_CUDA(cudaGetLastError());
-    return QDFN_OK;
-}
+int adj_local_blocks(int64_t RN) { return (int)((RN + kLocalThreads - 1) / kLocalThreads); }
 
 int adj_local(const AdjLocalArgs& a, cudaStream_t st) {
     const int64_t RN = (int64_t)a.R * a.N;
-    const int nblk = (int)((RN + kAdjThreads - 1) / kAdjThreads);
-    k_adj_local<<<nblk, kAdjThreads, 0, st>>>(a);
-    QDFN_CUDA(cudaGetLastError());
-    k_adj_sum_blocks<<<1, 32, 0, st>>>(nblk, a.R, a.blk_dt, a.blk_tx, a.sums);
+    k_adj_local<<<adj_local_blocks(RN), kLocalThreads, 0, st>>>(a);
     QDFN_CUDA(cudaGetLastError());
     return QDFN_OK;
 }
 
-int adj_local_blocks(int64_t RN) { return (int)((RN + kAdjThreads - 1) / kAdjThreads); }
-
-int adj_transpose(int prec, int R, const AdjTransArgs& a, const double* dloc, double* out, cudaStream_t st) {
+int adj_transpose(int prec, int R, const AdjTransArgs& a, const double* dloc, double* out, double* zero,
+                  cudaStream_t st) {
     switch (R) {
         case 1: launch_transpose_R<1>(prec, a, st); break;
         case 2: launch_transpose_R<2>(prec, a, st); break;
@@ -360,12 +398,13 @@ int adj_transpose(int prec, int R, const AdjTransArgs& a, const double* dloc, do
     }
     QDFN_CUDA(cudaGetLastError());
     const int64_t RN = (int64_t)R * a.N;
-    k_adj_combine<<<(unsigned)((RN + 255) / 256), 256, 0, st>>>(a.N, R, a.nrb, a.part, dloc, out);
+    k_adj_combine<<<(unsigned)((RN + 255) / 256), 256, 0, st>>>(a.N, R, a.nrb, a.part, dloc, out, zero);
     QDFN_CUDA(cudaGetLastError());
     return QDFN_OK;
 }
 
 int adj_transpose_prepare(int prec, int R, int64_t rpb) {
+    if (rpb != (prec == QDFN_FP64 ? 256 : 512)) return fail(QDFN_ERR_INVALID, "row block of the transposed product");
     const size_t sm = 2 * (size_t)R * rpb * (prec == QDFN_FP64 ? sizeof(double) : sizeof(float));
     if (sm > 48 * 1024) {
         cudaError_t e = cudaSuccess;
@@ -385,9 +424,8 @@ int adj_transpose_prepare(int prec, int R, int64_t rpb) {
     return QDFN_OK;
 }
 
-int adj_dtctl(int R, int64_t N, int64_t Ns, const double* V, const double* A, const unsigned char* unstable,
-              const int* has_unstable, double* out, cudaStream_t st) {
-    k_adj_dtctl<<<R, kAdjThreads, 0, st>>>(N, Ns, V, A, unstable, has_unstable, out);
+int adj_control(const AdjControlArgs& a, cudaStream_t st) {
+    k_adj_control<<<a.R, kCtlThreads, 0, st>>>(a);
     QDFN_CUDA(cudaGetLastError());
     return QDFN_OK;
 }

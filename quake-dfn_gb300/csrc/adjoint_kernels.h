@@ -29,7 +29,6 @@ struct AdjLocalArgs {
     double *oDloc, *oVold, *oThold, *oTLD, *oSig;
     double *ga, *gb, *gDc;             // parameter gradients, accumulated
     double *blk_dt, *blk_tx;           // [blocks][R] partial sums
-    double* sums;                      // [2R]: d/d(dt), d/d(external-stress time)
     int* err;                          // set when a residual's derivative vanishes
 };
 
@@ -45,10 +44,26 @@ struct AdjTransArgs {
 int adj_local(const AdjLocalArgs& a, cudaStream_t st);
 int adj_local_blocks(int64_t RN);
 int adj_transpose_prepare(int prec, int R, int64_t rpb);
-int adj_transpose(int prec, int R, const AdjTransArgs& a, const double* dloc, double* out, cudaStream_t st);
-// lV[idx[k]] += vals[k], lD[idx[k]] += vals[n + k], lA[idx[k]] += vals[2n + k] (device arrays)
-int adj_add(int n, const int64_t* idx, const double* vals, double* lV, double* lD, double* lA, cudaStream_t st);
-int adj_dtctl(int R, int64_t N, int64_t Ns, const double* V, const double* A, const unsigned char* unstable,
-              const int* has_unstable, double* out, cudaStream_t st);
+// out = dloc - E^T x_s + Kn^T x_n, and zero = 0
+int adj_transpose(int prec, int R, const AdjTransArgs& a, const double* dloc, double* out, double* zero,
+                  cudaStream_t st);
+
+// The adjoint of a reverse step's Dt and T, and the seeds of the state it ends
+// at (V null: the seeds alone, for the last state).
+struct AdjControlArgs {
+    int64_t N, Ns, state;              // the state's number in the window
+    int R, nblk, told;
+    double rupture_dt, max_dt, switch_v, dt_cut;
+    const double *V, *A;               // [R][N] the state the step's Dt was chosen from
+    const double *dt_now, *dt_prev;    // [R]
+    const unsigned char* unstable;
+    const int* has_unstable;
+    const double *blk_dt, *blk_tx;     // [nblk][R] from adj_local
+    double *lamT, *carry;              // [R], kept from step to step
+    const int64_t *seed_off, *seed_patch;   // [states * R + 1], [seeds]
+    const double* seed_val;            // [seeds][3]: dV, dD, dT
+    double *lV, *lD, *lA;
+};
+int adj_control(const AdjControlArgs& a, cudaStream_t st);
 
 }  // namespace qdfn

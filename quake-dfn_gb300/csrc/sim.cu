@@ -49,7 +49,6 @@ struct qdfn_ctx {
     double *la = nullptr, *lth0 = nullptr;   // ln(V_i/V0), ln(theta_i V0/Dc): F0's derivatives (adjoint)
     double* dref = nullptr;                   // [2][R] reference slip of the FP32/BF16 x copy
     double *rowsum_e = nullptr, *rowsum_n = nullptr;   // [N] row sums of the stored FP32/BF16 operator
-    unsigned char* sw_used = nullptr;         // adjoint recording: solver of each patch in the next launch
     double *ra = nullptr, *rDc = nullptr;
     unsigned char* unstable;
     int* has_unstable;
@@ -134,7 +133,6 @@ SimParams make_params(qdfn_ctx* c, uint64_t budget_ns) {
     SimParams p{};
     p.N = c->N; p.Nload = c->Nload; p.ld = c->ld; p.R = kernel_R(c->R);
     p.nblk = c->nblocks;
-    p.sw_used = c->sw_used;
     p.dref = c->dref;
     const bool offs = !c->hmat && c->prec != QDFN_FP64 && c->rowsum_e;
     p.rowsum_e = offs ? c->rowsum_e : nullptr;
@@ -616,39 +614,65 @@ extern "C" int qdfn_kernels_per_run(const qdfn_ctx* c) { return c ? 1 : 0; }
 // no derivatives): the reverse-mode gradient of a loss on the trajectory with
 // respect to the per-patch a, b and Dc.
 //
-// The forward window runs one step per launch and keeps the state every
-// `cp` steps (checkpoints, cp ~ sqrt(nsteps) by default).  The reverse sweep
-// takes the segments last to first: it restores the segment's checkpoint,
-// replays its steps one per launch recording each step's state, TLD, sigma
-// and solver (the tape), and walks the tape backwards.  Per step: the
-// per-patch vector-Jacobian products of the converged solves (adjoint.cuh,
-// FP64 dual numbers), the transposed stiffness products E^T and Kn^T over the
-// stored operator (FP32 or FP64, as in the forward), and the time step's
-// adjoint routed through the controller (Main_D :162-201): through the patch
-// that set min |V/Accel| / DtCut, through 1.2 x the previous step's Dt, or
-// nowhere (RuptureDt, MaximumDt); retried steps scale it by their halvings.
+// The forward window keeps the state every `cp` steps (checkpoints, cp ~
+// sqrt(nsteps) by default), one launch per segment.  The reverse sweep takes the
+// segments last to first: it restores the segment's checkpoint, replays its steps
+// in one launch recording each step's state, TLD, sigma and solver (the tape),
+// and walks the tape backwards.  A step of either launch runs as a launch of its
+// own would (SimParams::stepwise), so the segments' lengths change no bit.  Per
+// reverse step: the per-patch vector-Jacobian products of the converged solves
+// (adjoint.cuh), the transposed stiffness products E^T and Kn^T over the stored
+// operator (FP32 or FP64, as in the forward), and the time step's adjoint routed
+// through the controller (Main_D :162-201): through the patch that set
+// min |V/Accel| / DtCut, through 1.2 x the previous step's Dt, or nowhere
+// (RuptureDt, MaximumDt); retried steps scale it by their halvings.  The routing
+// runs on the device too (k_adj_control), so the sweep queues its steps without
+// the host in between.  3,001 patches, FP32, 36 steps: 12.7 ms with a launch per
+// step, a copy per taped field and three to five host round trips per reverse
+// step, 6.5 ms now.
 namespace {
 
+// One device allocation per call, cut into the call's buffers: a first pass
+// over the requests counts, the second hands out.
 struct DevMem {
-    std::vector<void*> ptrs;
+    unsigned char* base = nullptr;
+    size_t used = 0;
     template <class T>
-    int get(T** p, size_t n) {
+    void get(T** p, size_t n) {
+        *p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+    }
+    int alloc() {
+        const size_t n = used;
+        used = 0;
         void* q = nullptr;
-        if (cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess)
-            return fail(QDFN_ERR_NOMEM, "adjoint buffers");
-        ptrs.push_back(q);
-        *p = reinterpret_cast<T*>(q);
+        if (cudaMalloc(&q, n) != cudaSuccess) return fail(QDFN_ERR_NOMEM, "adjoint buffers");
+        base = reinterpret_cast<unsigned char*>(q);
         return QDFN_OK;
     }
     ~DevMem() {
-        for (void* q : ptrs) cudaFree(q);
+        if (base) cudaFree(base);
     }
 };
 
-// one launch of `nsteps` steps on st, as qdfn_run_async (no status check)
-int launch_steps(qdfn_ctx* c, int64_t nsteps, uint64_t budget_ns, cudaStream_t st) {
+// tape of one segment: states 0..cp, steps 1..cp
+struct Tape {
+    double *V, *D, *th, *A, *tld, *sig, *T, *dt;
+    unsigned char* sw;
+};
+
+// one launch of `nsteps` steps on st, each as a launch of its own would run it,
+// recorded on `tape` where given (no status check)
+int launch_steps(qdfn_ctx* c, int64_t nsteps, uint64_t budget_ns, const Tape* tape, cudaStream_t st) {
     QDFN_CUDA(cudaMemsetAsync(c->gerr, 0, 2 * sizeof(int), st));
     SimParams p = make_params(c, budget_ns);
+    p.stepwise = 1;
+    p.c_spec = 0;
+    if (tape) {
+        p.tape_V = tape->V; p.tape_D = tape->D; p.tape_th = tape->th; p.tape_A = tape->A;
+        p.tape_tld = tape->tld; p.tape_sig = tape->sig; p.tape_T = tape->T; p.tape_dt = tape->dt;
+        p.sw_used = tape->sw;
+    }
     SimKernel k = sim_kernel(c->prec, c->R, c->hmat != 0);
     void* args[] = {&p, &nsteps};
     QDFN_CUDA(cudaLaunchCooperativeKernel((const void*)k, dim3(c->nblocks), dim3(kSimThreads), args, c->smem, st));
@@ -716,184 +740,116 @@ extern "C" int qdfn_adjoint_run(qdfn_ctx* c, int64_t nsteps, int64_t checkpoint_
     const uint64_t budget_ns = (uint64_t)((timeout_s > 0 ? timeout_s : 1e6) * 1e9);
     cudaStream_t st = nullptr;
     int rc;
-    DevMem m;
     // checkpoints (nseg, the state before each segment) and the final state
     std::vector<Snap> ck(nseg + 1);
-    for (auto& k : ck)
-        if ((rc = m.get(&k.s6, 6 * RN)) || (rc = m.get(&k.Tdt, 2 * Rk)) || (rc = m.get(&k.step, Rk))) return rc;
-    // tape of one segment: state s = 0..cp (V, D, theta, accel), steps 1..cp (tld, sigma, solver), T and dt
-    double *tV, *tD, *tth, *tA, *ttld, *tsig, *tT, *tdt;
-    unsigned char* tsw;
-    if ((rc = m.get(&tV, (cp + 1) * RN)) || (rc = m.get(&tD, (cp + 1) * RN)) || (rc = m.get(&tth, (cp + 1) * RN)) ||
-        (rc = m.get(&tA, (cp + 1) * RN)) || (rc = m.get(&ttld, cp * RN)) || (rc = m.get(&tsig, cp * RN)) ||
-        (rc = m.get(&tsw, cp * RN)) || (rc = m.get(&tT, (cp + 1) * Rk)) || (rc = m.get(&tdt, (cp + 1) * Rk)))
-        return rc;
+    Tape tp;
     // adjoint state and work arrays
-    double *lV, *lD, *lth, *lA, *oDloc, *oVold, *oThold, *oTLD, *oSig, *ga, *gb, *gDc, *bdt, *btx, *sums, *part,
-        *ctl, *addv;
-    int64_t* addi;
+    double *lV, *lD, *lth, *lA, *oDloc, *oVold, *oThold, *oTLD, *oSig, *ga, *gb, *gDc, *bdt, *btx, *part, *lamT,
+        *carry, *seedv;
+    int64_t *seedk, *seedo;
     int* derr;
     const int nblk = adj_local_blocks(RN);
     const int64_t rpb = c->ld, nrb = (N + rpb - 1) / rpb;
-    const int64_t max_add = std::max<int64_t>(n_seeds + Rk, 1);
-    if ((rc = m.get(&lV, RN)) || (rc = m.get(&lD, RN)) || (rc = m.get(&lth, RN)) || (rc = m.get(&lA, RN)) ||
-        (rc = m.get(&oDloc, RN)) || (rc = m.get(&oVold, RN)) || (rc = m.get(&oThold, RN)) ||
-        (rc = m.get(&oTLD, RN)) || (rc = m.get(&oSig, RN)) || (rc = m.get(&ga, RN)) || (rc = m.get(&gb, RN)) ||
-        (rc = m.get(&gDc, RN)) || (rc = m.get(&bdt, (int64_t)nblk * Rk)) || (rc = m.get(&btx, (int64_t)nblk * Rk)) ||
-        (rc = m.get(&sums, 2 * Rk)) || (rc = m.get(&part, nrb * 2 * RN)) || (rc = m.get(&ctl, 5 * Rk)) ||
-        (rc = m.get(&addv, 3 * max_add)) || (rc = m.get(&addi, max_add)) || (rc = m.get(&derr, 1)))
-        return rc;
+    DevMem m;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (auto& k : ck) { m.get(&k.s6, 6 * RN); m.get(&k.Tdt, 2 * Rk); m.get(&k.step, Rk); }
+        m.get(&tp.V, (cp + 1) * RN); m.get(&tp.D, (cp + 1) * RN); m.get(&tp.th, (cp + 1) * RN);
+        m.get(&tp.A, (cp + 1) * RN); m.get(&tp.tld, cp * RN); m.get(&tp.sig, cp * RN); m.get(&tp.sw, cp * RN);
+        m.get(&tp.T, (cp + 1) * Rk); m.get(&tp.dt, (cp + 1) * Rk);
+        m.get(&lV, RN); m.get(&lD, RN); m.get(&lth, RN); m.get(&lA, RN); m.get(&oDloc, RN); m.get(&oVold, RN);
+        m.get(&oThold, RN); m.get(&oTLD, RN); m.get(&oSig, RN); m.get(&ga, RN); m.get(&gb, RN); m.get(&gDc, RN);
+        m.get(&bdt, (int64_t)nblk * Rk); m.get(&btx, (int64_t)nblk * Rk); m.get(&part, nrb * 2 * RN);
+        m.get(&lamT, Rk); m.get(&carry, Rk); m.get(&seedv, 3 * n_seeds); m.get(&seedk, n_seeds);
+        m.get(&seedo, (nsteps + 2) * Rk); m.get(&derr, 1);
+        if (pass == 0 && (rc = m.alloc())) return rc;
+    }
     if ((rc = adj_transpose_prepare(c->prec, Rk, rpb))) return rc;
     for (double* z : {lV, lD, lth, lA, ga, gb, gDc}) QDFN_CUDA(cudaMemsetAsync(z, 0, RN * 8, st));
+    for (double* z : {lamT, carry}) QDFN_CUDA(cudaMemsetAsync(z, 0, Rk * 8, st));
     QDFN_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), st));
 
-    // ---- forward: one step per launch, a checkpoint every cp steps
+    // ---- forward: a checkpoint before each segment
     for (int64_t seg = 0; seg < nseg; ++seg) {
         if ((rc = snap_save(c, ck[seg], st))) return rc;
-        const int64_t len = std::min(cp, nsteps - seg * cp);
-        for (int64_t t = 0; t < len; ++t)
-            if ((rc = launch_steps(c, 1, budget_ns, st))) return rc;
+        if ((rc = launch_steps(c, std::min(cp, nsteps - seg * cp), budget_ns, nullptr, st))) return rc;
         if ((rc = run_status(c, st))) return rc;
     }
     if ((rc = snap_save(c, ck[nseg], st))) return rc;
 
-    // ---- seeds by step
-    std::vector<std::vector<int64_t>> by_step(nsteps + 1);
-    for (int64_t k = 0; k < n_seeds; ++k) by_step[seed_step[k]].push_back(k);
-    std::vector<double> lamT(Rk, 0.0), carry(Rk, 0.0);
+    // ---- seeds by (step, instance), in their order: patch (-1: time alone), then dV, dD, dT
+    {
+        std::vector<int64_t> off((nsteps + 2) * Rk, 0), key(n_seeds);
+        std::vector<double> val(3 * n_seeds);
+        for (int64_t k = 0; k < n_seeds; ++k) off[seed_step[k] * Rk + seed_inst[k] + 1]++;
+        for (size_t k = 1; k < off.size(); ++k) off[k] += off[k - 1];
+        std::vector<int64_t> at(off);
+        for (int64_t k = 0; k < n_seeds; ++k) {
+            const int64_t o = at[seed_step[k] * Rk + seed_inst[k]]++;
+            key[o] = seed_patch[k];
+            val[3 * o] = seed_dV[k]; val[3 * o + 1] = seed_dD[k]; val[3 * o + 2] = seed_dT[k];
+        }
+        QDFN_CUDA(cudaMemcpy(seedo, off.data(), off.size() * 8, cudaMemcpyHostToDevice));
+        if (n_seeds) {
+            QDFN_CUDA(cudaMemcpy(seedk, key.data(), n_seeds * 8, cudaMemcpyHostToDevice));
+            QDFN_CUDA(cudaMemcpy(seedv, val.data(), 3 * n_seeds * 8, cudaMemcpyHostToDevice));
+        }
+    }
     if (dL_dD_final) {
         std::vector<double> h(RN, 0.0);
         std::memcpy(h.data(), dL_dD_final, (size_t)R * N * 8);
         QDFN_CUDA(cudaMemcpy(lD, h.data(), RN * 8, cudaMemcpyHostToDevice));
     }
-    // adds seeds of state n and controller terms to (lV, lD, lA), lamT
-    std::vector<int64_t> hi;
-    std::vector<double> hv;
-    auto apply_adds = [&](const std::vector<int64_t>& idx, const std::vector<double>& vV,
-                          const std::vector<double>& vD, const std::vector<double>& vA) -> int {
-        const int n = (int)idx.size();
-        if (n == 0) return QDFN_OK;
-        std::vector<double> v(3 * (size_t)n);
-        for (int k = 0; k < n; ++k) { v[k] = vV[k]; v[n + k] = vD[k]; v[2 * n + k] = vA[k]; }
-        QDFN_CUDA(cudaMemcpy(addi, idx.data(), n * 8, cudaMemcpyHostToDevice));
-        QDFN_CUDA(cudaMemcpy(addv, v.data(), 3 * (size_t)n * 8, cudaMemcpyHostToDevice));
-        return adj_add(n, addi, addv, lV, lD, lA, st);
-    };
-    auto seeds_of = [&](int64_t n) -> int {
-        std::vector<int64_t> idx;
-        std::vector<double> vV, vD, vA;
-        for (int64_t k : by_step[n]) {
-            lamT[seed_inst[k]] += seed_dT[k];
-            if (seed_patch[k] >= 0) {
-                idx.push_back((int64_t)seed_inst[k] * N + seed_patch[k]);
-                vV.push_back(seed_dV[k]); vD.push_back(seed_dD[k]); vA.push_back(0.0);
-            }
-        }
-        return apply_adds(idx, vV, vD, vA);
-    };
-    if ((rc = seeds_of(nsteps))) return rc;
+    AdjControlArgs ca{};
+    ca.N = N; ca.Ns = Ns; ca.R = Rk; ca.nblk = nblk;
+    ca.told = c->prob.interp_at_told != 0; ca.rupture_dt = c->prob.rupture_dt; ca.max_dt = c->prob.max_dt;
+    ca.switch_v = c->prob.switch_v; ca.dt_cut = c->prob.dt_cut;
+    ca.unstable = c->unstable; ca.has_unstable = c->has_unstable; ca.blk_dt = bdt; ca.blk_tx = btx;
+    ca.lamT = lamT; ca.carry = carry; ca.seed_off = seedo; ca.seed_patch = seedk; ca.seed_val = seedv;
+    ca.lV = lV; ca.lD = lD; ca.lA = lA; ca.state = nsteps;
+    if ((rc = adj_control(ca, st))) return rc;   // the seeds of the last state
 
-    const double rupture = c->prob.rupture_dt, maxdt = c->prob.max_dt, swv = c->prob.switch_v, dtcut = c->prob.dt_cut;
-    const bool told = c->prob.interp_at_told != 0;
     // ---- reverse, segment by segment
     for (int64_t seg = nseg - 1; seg >= 0; --seg) {
         const int64_t s0 = seg * cp, len = std::min(cp, nsteps - s0);
         if ((rc = snap_load(c, ck[seg], st))) return rc;
-        auto rec_state = [&](int64_t t) -> int {   // tape state t from the context's host-visible state
-            QDFN_CUDA(cudaMemcpyAsync(tV + t * RN, c->V, RN * 8, cudaMemcpyDeviceToDevice, st));
-            QDFN_CUDA(cudaMemcpyAsync(tD + t * RN, c->D, RN * 8, cudaMemcpyDeviceToDevice, st));
-            QDFN_CUDA(cudaMemcpyAsync(tth + t * RN, c->theta, RN * 8, cudaMemcpyDeviceToDevice, st));
-            QDFN_CUDA(cudaMemcpyAsync(tA + t * RN, c->accel, RN * 8, cudaMemcpyDeviceToDevice, st));
-            QDFN_CUDA(cudaMemcpyAsync(tT + t * Rk, c->T, Rk * 8, cudaMemcpyDeviceToDevice, st));
-            QDFN_CUDA(cudaMemcpyAsync(tdt + t * Rk, c->dt, Rk * 8, cudaMemcpyDeviceToDevice, st));
-            return QDFN_OK;
-        };
-        if ((rc = rec_state(0))) return rc;
-        for (int64_t t = 1; t <= len; ++t) {
-            c->sw_used = tsw + (t - 1) * RN;
-            rc = launch_steps(c, 1, budget_ns, st);
-            c->sw_used = nullptr;
-            if (rc) return rc;
-            if ((rc = rec_state(t))) return rc;
-            QDFN_CUDA(cudaMemcpyAsync(ttld + (t - 1) * RN, c->tld, RN * 8, cudaMemcpyDeviceToDevice, st));
-            QDFN_CUDA(cudaMemcpyAsync(tsig + (t - 1) * RN, c->sig_old, RN * 8, cudaMemcpyDeviceToDevice, st));
-        }
+        // tape state 0 from the checkpoint (its fields: V, D, theta, friction, accel, sigma)
+        const double* s6 = ck[seg].s6;
+        QDFN_CUDA(cudaMemcpyAsync(tp.V, s6, RN * 8, cudaMemcpyDeviceToDevice, st));
+        QDFN_CUDA(cudaMemcpyAsync(tp.D, s6 + RN, RN * 8, cudaMemcpyDeviceToDevice, st));
+        QDFN_CUDA(cudaMemcpyAsync(tp.th, s6 + 2 * RN, RN * 8, cudaMemcpyDeviceToDevice, st));
+        QDFN_CUDA(cudaMemcpyAsync(tp.A, s6 + 4 * RN, RN * 8, cudaMemcpyDeviceToDevice, st));
+        QDFN_CUDA(cudaMemcpyAsync(tp.T, ck[seg].Tdt, Rk * 8, cudaMemcpyDeviceToDevice, st));
+        QDFN_CUDA(cudaMemcpyAsync(tp.dt, ck[seg].Tdt + Rk, Rk * 8, cudaMemcpyDeviceToDevice, st));
+        if ((rc = launch_steps(c, len, budget_ns, &tp, st))) return rc;
         if ((rc = run_status(c, st))) return rc;
-        std::vector<double> hdt((len + 1) * Rk), hT((len + 1) * Rk);
-        QDFN_CUDA(cudaMemcpy(hdt.data(), tdt, hdt.size() * 8, cudaMemcpyDeviceToHost));
-        QDFN_CUDA(cudaMemcpy(hT.data(), tT, hT.size() * 8, cudaMemcpyDeviceToHost));
-        for (int64_t t = len; t >= 1; --t) {
-            const int64_t n = s0 + t;   // the step taking tape state t-1 to t
+        for (int64_t t = len; t >= 1; --t) {   // the step taking tape state t-1 to t
             AdjLocalArgs a{};
-            a.N = N; a.Ns = Ns; a.R = Rk; a.dr = c->prob.evolution_dr; a.interp_at_told = told ? 1 : 0;
+            a.N = N; a.Ns = Ns; a.R = Rk; a.dr = c->prob.evolution_dr; a.interp_at_told = ca.told ? 1 : 0;
             a.eta = c->eta; a.sigma_min = c->prob.sigma_min;
-            a.Vprev = tV + (t - 1) * RN; a.Dprev = tD + (t - 1) * RN; a.thprev = tth + (t - 1) * RN;
-            a.Vcur = tV + t * RN; a.tld = ttld + (t - 1) * RN; a.sig = tsig + (t - 1) * RN;
-            a.sw = tsw + (t - 1) * RN;
-            a.dt = tdt + t * Rk; a.Tprev = tT + (t - 1) * Rk;
+            a.Vprev = tp.V + (t - 1) * RN; a.Dprev = tp.D + (t - 1) * RN; a.thprev = tp.th + (t - 1) * RN;
+            a.Vcur = tp.V + t * RN; a.tld = tp.tld + (t - 1) * RN; a.sig = tp.sig + (t - 1) * RN;
+            a.sw = tp.sw + (t - 1) * RN;
+            a.dt = tp.dt + t * Rk; a.Tprev = tp.T + (t - 1) * Rk;
             a.pa = c->a; a.pb = c->b; a.pDc = c->Dc; a.F0 = c->F0; a.la = c->la; a.lth0 = c->lth0;
             a.kself = c->kself; a.mass = c->mass; a.omega = c->omega; a.tau0 = c->tau0;
             a.n_ext = c->n_ext; a.ext_t = c->ext_t; a.ext_n = c->ext_n; a.ext_s = c->ext_s; a.ext_p = c->ext_p;
             a.lV = lV; a.lD = lD; a.lth = lth; a.lA = lA;
             a.oDloc = oDloc; a.oVold = oVold; a.oThold = oThold; a.oTLD = oTLD; a.oSig = oSig;
-            a.ga = ga; a.gb = gb; a.gDc = gDc; a.blk_dt = bdt; a.blk_tx = btx; a.sums = sums; a.err = derr;
+            a.ga = ga; a.gb = gb; a.gDc = gDc; a.blk_dt = bdt; a.blk_tx = btx; a.err = derr;
             if ((rc = adj_local(a, st))) return rc;
             AdjTransArgs tr{};
             tr.N = N; tr.rpb = rpb; tr.nrb = nrb; tr.gx = std::max<int64_t>(1, (4 * num_sms() + nrb - 1) / nrb);
             tr.E = c->E; tr.Kn = c->Kn; tr.x_s = oTLD; tr.x_n = oSig; tr.part = part;
-            if ((rc = adj_transpose(c->prec, Rk, tr, oDloc, lD, st))) return rc;   // lambda_D of state t-1
+            // lambda_D of state t-1; its lambda_Accel starts at zero
+            if ((rc = adj_transpose(c->prec, Rk, tr, oDloc, lD, lA, st))) return rc;
             std::swap(lV, oVold);
             std::swap(lth, oThold);
-            QDFN_CUDA(cudaMemsetAsync(lA, 0, RN * 8, st));
-            if ((rc = adj_dtctl(Rk, N, Ns, tV + (t - 1) * RN, tA + (t - 1) * RN, c->unstable, c->has_unstable, ctl,
-                                st)))
-                return rc;
-            std::vector<double> hs(2 * Rk), hc(5 * Rk);
-            QDFN_CUDA(cudaMemcpyAsync(hs.data(), sums, hs.size() * 8, cudaMemcpyDeviceToHost, st));
-            QDFN_CUDA(cudaMemcpyAsync(hc.data(), ctl, hc.size() * 8, cudaMemcpyDeviceToHost, st));
-            QDFN_CUDA(cudaStreamSynchronize(st));
-            // the step's dt: its patches, T_n = T_{n-1} + dt, the external-stress
-            // time (TOld + Dt in main, TOld in main_H), the next step's 1.2 Dt
-            std::vector<int64_t> idx;
-            std::vector<double> vV, vD, vA;
-            for (int r = 0; r < Rk; ++r) {
-                const double ldt = hs[r] + lamT[r] + (told ? 0.0 : hs[Rk + r]) + carry[r];
-                lamT[r] += hs[Rk + r];
-                carry[r] = 0.0;
-                // the controller that chose this step's Dt, from state t-1
-                const double dtn = hdt[t * Rk + r], dtp = hdt[(t - 1) * Rk + r];
-                double vmax = hc[r * 5 + 0];
-                if (hc[r * 5 + 1] != 0) vmax = NAN;
-                const double dtmin = hc[r * 5 + 2] / dtcut;
-                const bool usable = hc[r * 5 + 3] != 0;
-                int src = 0;   // 0 constant, 1 min |V/A| / DtCut, 2 1.2 x previous Dt
-                double ref;
-                if (vmax > swv) ref = rupture;
-                else if (dtmin > maxdt) ref = maxdt;
-                else { ref = dtmin; src = usable ? 1 : 0; }
-                double dtc;
-                if (ref <= rupture) dtc = ref;
-                else if (dtp < ref / 1.2) { dtc = dtp * 1.2; src = 2; }
-                else dtc = ref;
-                const double sc = dtn / dtc;
-                const double e2 = std::log2(sc);
-                if (!(sc > 0 && sc <= 1 && std::fabs(e2 - std::round(e2)) < 1e-9)) src = 0;   // e.g. Dt = 1e-3
-                if (src == 1) {
-                    const int64_t k = (int64_t)hc[r * 5 + 4];
-                    double Vk = 0, Ak = 0;
-                    QDFN_CUDA(cudaMemcpy(&Vk, tV + (t - 1) * RN + (int64_t)r * N + k, 8, cudaMemcpyDeviceToHost));
-                    QDFN_CUDA(cudaMemcpy(&Ak, tA + (t - 1) * RN + (int64_t)r * N + k, 8, cudaMemcpyDeviceToHost));
-                    const double q = Vk / Ak, sg = q < 0 ? -1.0 : 1.0;
-                    idx.push_back((int64_t)r * N + k);
-                    vV.push_back(ldt * sc * sg / (Ak * dtcut));
-                    vD.push_back(0.0);
-                    vA.push_back(-ldt * sc * sg * Vk / (Ak * Ak * dtcut));
-                } else if (src == 2) {
-                    carry[r] = 1.2 * sc * ldt;
-                }
-            }
-            if ((rc = apply_adds(idx, vV, vD, vA))) return rc;
-            if ((rc = seeds_of(n - 1))) return rc;
+            // the step's dt, T_n = T_{n-1} + dt, the external-stress time (TOld + Dt
+            // in main, TOld in main_H), the next step's 1.2 Dt; then state t-1's seeds
+            ca.V = tp.V + (t - 1) * RN; ca.A = tp.A + (t - 1) * RN;
+            ca.dt_now = tp.dt + t * Rk; ca.dt_prev = tp.dt + (t - 1) * Rk;
+            ca.lV = lV; ca.state = s0 + t - 1;
+            if ((rc = adj_control(ca, st))) return rc;
         }
     }
     int herr = 0;

@@ -136,8 +136,15 @@ struct SimParams {
     // have, so that no SM idles while the slowest member finishes
     unsigned* fill_ctr;
     unsigned fill_need;
-    // adjoint recording (null: off): the solver each patch's accepted pass
-    // used, [R][N] (0 low velocity, 1 high velocity, 2 loading fault)
+    // adjoint windows.  stepwise: every step of the launch runs as if it were a
+    // launch of its own -- the FP32/BF16 x copy is formed anew from the state with
+    // its own offset -- so that a window's steps do not depend on how it is cut
+    // into launches (with c_spec = 0).  tape (tape_V null: off): the state after
+    // step k of the launch at [k + 1][R][N], and of step k at [k][R][N] the
+    // stress products, sigma and the solver each patch's accepted pass used
+    // (0 low velocity, 1 high velocity, 2 loading fault)
+    int stepwise;
+    double *tape_V, *tape_D, *tape_th, *tape_A, *tape_tld, *tape_sig, *tape_T, *tape_dt;
     unsigned char* sw_used;
     // FP32/BF16 dense operator: the x copy of D holds D - dref (dref = slip of
     // patch 0 at the start of the step before, per instance, [2][R] by step
@@ -1235,6 +1242,18 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
         const bool offs = !HM && sizeof(X) == 4 && p.rowsum_e != nullptr;
         if (offs && blk == 0 && threadIdx.x < R)
             p.dref[((it + 1) & 1) * R + threadIdx.x] = (par ? p.Dn : p.D)[(int64_t)threadIdx.x * N];
+        if (offs && p.stepwise && it > 0) {   // the x copy with this step's own offset
+            const double* Dc = par ? p.Dn : p.D;
+            X* x = reinterpret_cast<X*>(p.xd) + (size_t)par * p.xd_stride;
+            for (int64_t q = gtid; q < (int64_t)R * N; q += nthreads) {
+                const int r = (int)(q / N);
+                const int64_t i = q - (int64_t)r * N;
+                x[i * R + r] = (X)(Dc[q] - Dc[(int64_t)r * N]);
+            }
+            fence_proxy_async_global();
+            if (blk == 0 && threadIdx.x < R) p.dref[(it & 1) * R + threadIdx.x] = Dc[(int64_t)threadIdx.x * N];
+            if (!grid_barrier(p, deadline)) return;
+        }
         const int cpar = (int)(it % kSets);   // which counter set this step uses
         const int cnext = (int)((it + 1) % kSets);
         if (threadIdx.x < R) s_done[threadIdx.x] = 0;
@@ -1326,7 +1345,10 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                     o = sim::solve_reference(pin, swq == 1, pair, Dt, p.eta, p.alpha_evo, p.evolution_dr, p.switch_v, err);
                 if (!writer) return;
                 if (!HM && first) { p.tld[q] = tld_q; p.knd[q] = knd_q; }
-                if (p.sw_used) p.sw_used[q] = (unsigned char)swq;
+                if (p.tape_V) {
+                    p.tape_tld[it * R * N + q] = tld_q;
+                    p.sw_used[it * R * N + q] = (unsigned char)swq;
+                }
                 QDFN_NXT(V, Vn)[q] = o.V; QDFN_NXT(fric, fn)[q] = o.Friction; QDFN_NXT(D, Dn)[q] = o.Disp;
                 QDFN_NXT(theta, thn)[q] = o.Theta; QDFN_NXT(sig_old, sn)[q] = sig;
                 p.dtall[q] = o.Dt; p.instab[q] = o.Instab; p.flag[q] = o.Flag;
@@ -1348,7 +1370,10 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
             } else {
                 if (!writer) return;   // loading faults (Solvers :370-377)
                 if (!HM && first) { p.tld[q] = tld_q; p.knd[q] = knd_q; }
-                if (p.sw_used) p.sw_used[q] = 2;
+                if (p.tape_V) {
+                    p.tape_tld[it * R * N + q] = tld_q;
+                    p.sw_used[it * R * N + q] = 2;
+                }
                 const double Vc = p.Vconst[q];
                 const double Dn = QDFN_CUR(D, Dn)[q] + Vc * Dt;
                 QDFN_NXT(V, Vn)[q] = Vc; QDFN_NXT(fric, fn)[q] = QDFN_CUR(fric, fn)[q]; QDFN_NXT(D, Dn)[q] = Dn;
@@ -1792,6 +1817,19 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
                         }
                     }
                 }
+            }
+        }
+        if (p.tape_V) {
+            const StateView nxt = state_view(p, par ^ 1);
+            const int64_t o = (it + 1) * R * N;
+            for (int64_t q = gtid; q < (int64_t)R * N; q += nthreads) {
+                p.tape_V[o + q] = nxt.V[q]; p.tape_D[o + q] = nxt.D[q]; p.tape_th[o + q] = nxt.theta[q];
+                p.tape_A[o + q] = nxt.accel[q];
+                p.tape_sig[it * R * N + q] = nxt.sig_old[q];
+            }
+            if (blk == 0 && threadIdx.x < R) {
+                p.tape_T[(it + 1) * R + threadIdx.x] = s_T[threadIdx.x] + s_dt[threadIdx.x];
+                p.tape_dt[(it + 1) * R + threadIdx.x] = s_dt[threadIdx.x];
             }
         }
         __syncthreads();
