@@ -11,14 +11,12 @@
 namespace qdfn {
 namespace {
 
-// one thread per member: error flag and barrier arrivals (adjacent words);
-// thread 0 also clears the fill-mode counter
-__global__ void k_members_reset(const SimParams* __restrict__ members, int n, unsigned* fill) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m == 0 && fill) *fill = 0u;
-    if (m >= n) return;
-    members[m].gerr[0] = 0;
-    *members[m].bar_count = 0u;
+// one block per member: its control words, from the error flag on; the first
+// also clears the fill-mode counter
+__global__ void k_members_reset(const SimParams* __restrict__ members, unsigned* fill) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && fill) *fill = 0u;
+    int* ctrl = members[blockIdx.x].gerr;
+    for (int k = threadIdx.x; k < (int)(kCtrlBytes / sizeof(int)); k += blockDim.x) ctrl[k] = 0;
 }
 
 // one thread per member: the first failing instance's status, else the
@@ -74,7 +72,7 @@ MembersKernel members_kernel(int prec, int R) {
 }
 
 int members_reset(const SimParams* dmembers, int n, unsigned* dfill, cudaStream_t st) {
-    k_members_reset<<<(n + 127) / 128, 128, 0, st>>>(dmembers, n, dfill);
+    k_members_reset<<<n, 128, 0, st>>>(dmembers, dfill);
     QDFN_CUDA(cudaGetLastError());
     return QDFN_OK;
 }

@@ -56,13 +56,13 @@ struct qdfn_ctx {
     int *instab, *flag, *sw, *sw_n;
     double* accel_n;
     double *part_s = nullptr, *part_n = nullptr;
-    size_t part_cap = 0, partn_cap = 0, red_cap = 0, xd_cap = 0;   // elements held by the work buffers
+    size_t part_cap = 0, partn_cap = 0, xd_cap = 0;   // elements held by the work buffers
     double *T, *dt;
     int64_t *step, *nrec;
     int* status;
     double *hT, *hDt, *hV, *hD, *hth, *hs;
     unsigned *bar_count, *bar_gen;
-    double* red = nullptr;
+    unsigned long long* red;
     int* gerr;
     unsigned long long* prof;
     unsigned long long* tile_ctr;
@@ -331,7 +331,6 @@ int configure_launch(qdfn_ctx* c) {
         if ((rc = ensure(&c->part_s, 2 * (size_t)c->part_stride, c->part_cap))) return rc;
         if ((rc = ensure(&c->part_n, 2 * (size_t)c->part_stride, c->partn_cap))) return rc;
     }
-    if ((rc = ensure(&c->red, (size_t)2 * c->nblocks * Rk * kRedSlots, c->red_cap))) return rc;
     return QDFN_OK;
 }
 
@@ -377,13 +376,15 @@ extern "C" int qdfn_ctx_create(qdfn_ctx** out, const qdfn_problem* pr) {
     const size_t hr = (size_t)Rk * std::max<int64_t>(pr->max_records, 1);
     A(hT, hr); A(hDt, hr); A(hV, hr * N); A(hD, hr * N); A(hth, hr * N); A(hs, hr * N);
     // launch control words side by side: [0] error flag, [1] barrier arrivals,
-    // [2] barrier generation -- the first two are cleared by one memset per launch
+    // [2] barrier generation, and from the second line the reductions' words --
+    // all cleared by one memset per launch
     int* ctrl = nullptr;
-    if (!rc) rc = c->dalloc(&ctrl, 4);
+    if (!rc) rc = c->dalloc(&ctrl, kCtrlBytes / sizeof(int));
     if (!rc) {
         c->gerr = ctrl;
         c->bar_count = reinterpret_cast<unsigned*>(ctrl + 1);
         c->bar_gen = reinterpret_cast<unsigned*>(ctrl + 2);
+        c->red = reinterpret_cast<unsigned long long*>(ctrl + 32);
     }
     A(prof, kCounters); A(tile_ctr, kSets); A(spec_ctr, kSets);
     // per-step counters, kSets sets used by steps in turn (a step uses one, streams
@@ -588,7 +589,7 @@ extern "C" int qdfn_run_async(qdfn_ctx* c, int64_t nsteps, double timeout_s, voi
     const uint64_t budget_ns = (uint64_t)(budget * 1e9);
     cudaStream_t st = (cudaStream_t)stream;
     // error flag and barrier arrivals (adjacent); the kernel resets its own counters
-    QDFN_CUDA(cudaMemsetAsync(c->gerr, 0, 2 * sizeof(int), st));
+    QDFN_CUDA(cudaMemsetAsync(c->gerr, 0, kCtrlBytes, st));
     SimParams p = make_params(c, budget_ns);
     SimKernel k = sim_kernel(c->prec, c->R, c->hmat != 0);
     void* args[] = {&p, &nsteps};
@@ -676,7 +677,7 @@ struct Tape {
 // one launch of `nsteps` steps on st, each as a launch of its own would run it,
 // recorded on `tape` where given (no status check)
 int launch_steps(qdfn_ctx* c, int64_t nsteps, uint64_t budget_ns, const Tape* tape, cudaStream_t st) {
-    QDFN_CUDA(cudaMemsetAsync(c->gerr, 0, 2 * sizeof(int), st));
+    QDFN_CUDA(cudaMemsetAsync(c->gerr, 0, kCtrlBytes, st));
     SimParams p = make_params(c, budget_ns);
     p.stepwise = 1;
     p.c_spec = 0;
