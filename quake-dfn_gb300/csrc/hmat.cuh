@@ -75,10 +75,22 @@ __device__ __forceinline__ int64_t snake_task(int64_t k, int64_t w, int64_t W) {
     return k * W + ((k & 1) ? W - 1 - w : w);
 }
 
-// rank rows per pass-A task: each lane keeps (hi, lo) sums for every row and
-// instance in registers
-template <int R>
-__host__ __device__ constexpr int rows_a() { return R <= 2 ? 8 : 4; }
+// rank rows per pass-A task of a short block: each lane keeps (hi, lo) sums for
+// every row and instance in registers
+__host__ __device__ constexpr int rows_a(int R) { return R <= 2 ? 8 : 4; }
+// and its 32-column rounds per batch (rows x rounds loads per lane in flight,
+// within the persistent kernel's 128 registers)
+__host__ __device__ constexpr int rounds_a(int R, int elem) { return elem == 4 && R == 1 ? 4 : 2; }
+// A block with many sources gives its tasks half or a quarter of the rows and
+// batches twice or four times as long: the same loads in flight and a shorter chain
+// of batches.  (One task of the largest block took 32 us, the average warp had 12
+// us of pass A.  6,000 triangles, us a step for the two passes: 46 -> 37, FP64 182
+// -> 108, two instances 63 -> 48.  With four the loads of x outnumber the rows':
+// 84 -> 91, so not there.)
+__host__ __device__ constexpr int level_a(int64_t ns, int R, int elem) {
+    const int64_t batch = 32 * rounds_a(R, elem);
+    return R > 2 || ns <= 2 * batch ? 0 : ns <= 8 * batch ? 1 : 2;
+}
 
 // A task's block descriptor, loaded once per task: nine independent 8-byte
 // loads (every lane the same words; the array's 72-byte stride keeps only
@@ -94,7 +106,7 @@ __device__ __forceinline__ Blk load_blk(const Blk* p) {
     return b;
 }
 
-// Warp sums of G values per lane (G = 4 or 8; R instances each) kept as FP32
+// Warp sums of G values per lane (G = 1 to 8; R instances each) kept as FP32
 // (hi, lo) pairs (FP64 storage: hi alone).  The first log2(G) butterfly levels
 // halve the values a lane holds -- at offset o a lane keeps the half its lane
 // bit o selects and adds its partner's copy of that half -- so that lane L
@@ -106,7 +118,7 @@ __device__ __forceinline__ Blk load_blk(const Blk* p) {
 // L % (32 / G) == 0); fixed order, so results are reproducible.
 template <class T, int G, int R>
 __device__ __forceinline__ void warp_sums(T (&hi)[G][R], T (&lo)[G][R], int lane, double (&out)[R]) {
-    static_assert(G == 4 || G == 8, "rank rows per task");
+    static_assert(G == 1 || G == 2 || G == 4 || G == 8, "rank rows per task");
     auto combine = [](T& ah, T& al, T bh, T bl) {
         if constexpr (sizeof(T) == 4) {
             const T s = ah + bh, bp = s - ah;
@@ -160,21 +172,69 @@ __device__ __forceinline__ BlkA load_blk_a(const Blk* p) {
     return b;
 }
 
+// One pass-A task: up to G rank rows of block b from kk0 on, batches of UA 32-column
+// rounds
+template <class T, int G, int UA, int R>
+__device__ __forceinline__ void task_a(const Ops& h, const double* __restrict__ D, int64_t N, const BlkA& b, int kk0) {
+    const int lane = threadIdx.x & 31;
+    const int nrow = min(G, b.rank - kk0);
+    const T* row0 = reinterpret_cast<const T*>(h.store) + b.off_a + (int64_t)kk0 * b.ns;
+    const double* xs = D + b.s0;
+    // each lane's products summed in T -- FP32 storage as an error-free
+    // (hi, lo) pair on the FP32 pipe -- then the warp's sums (warp_sums)
+    T hi[G][R], lo[G][R];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int r = 0; r < R; ++r) { hi[g][r] = 0; lo[g][r] = 0; }
+    for (int64_t j0 = 0; j0 < b.ns; j0 += 32 * UA) {
+        T v[UA][G], xv[UA][R];
+#pragma unroll
+        for (int u = 0; u < UA; ++u) {
+            const int64_t j = j0 + u * 32 + lane;
+            const bool ok = j < b.ns;
+#pragma unroll
+            for (int g = 0; g < G; ++g) v[u][g] = (ok && g < nrow) ? __ldg(row0 + (int64_t)g * b.ns + j) : (T)0;
+#pragma unroll
+            for (int r = 0; r < R; ++r) xv[u][r] = ok ? (T)__ldcg(xs + (int64_t)r * N + j) : (T)0;
+        }
+#pragma unroll
+        for (int u = 0; u < UA; ++u)
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const T pr = v[u][g] * xv[u][r];
+                    if constexpr (sizeof(T) == 4) {
+                        const T sum = hi[g][r] + pr, bp = sum - hi[g][r];
+                        lo[g][r] += (hi[g][r] - (sum - bp)) + (pr - bp);
+                        hi[g][r] = sum;
+                    } else {
+                        hi[g][r] += pr;
+                    }
+                }
+    }
+    double tot[R];
+    warp_sums<T, G, R>(hi, lo, lane, tot);
+    constexpr int kSpan = 32 / G;   // lanes per row after the halving levels
+    const int g = lane / kSpan;
+    if (lane % kSpan == 0 && g < nrow) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) h.t[(b.toff + kk0 + g) * R + r] = tot[r];
+    }
+}
+
 // pass A: t_b = Vt_b x[src], one task per (low-rank block, group of up to
-// rows_a rank rows): the lanes stride the block's source range, each load of
-// x serving every row of the group, and each round issues the group's rows x 4
+// rows_a rank rows, fewer of long blocks): the lanes stride the block's source range, each load of
+// x serving every row of the group, and each batch issues the group's rows x 4
 // column loads before any of them is used (HBM latency is hidden by the loads
 // in flight, not by occupancy: one 16-warp CTA per SM).  Out of line, like pass
 // B: beside the inlined solvers the loops lost registers and loads in flight
 // (6,000 triangles: the two passes 51 us a step, 42 out of line).
 template <class T, int R>
 __device__ __noinline__ void pass_a(const Ops h, const double* __restrict__ D, int64_t N, T*, double*) {
-    constexpr int G = rows_a<R>();
-    // 32-column rounds per batch (G x kUA loads per lane in flight), within the
-    // persistent kernel's 128 registers
-    constexpr int kUA = (sizeof(T) == 4 && R == 1) ? 4 : 2;
+    constexpr int G = rows_a(R), UA = rounds_a(R, sizeof(T));
     const int lane = threadIdx.x & 31;
-    const T* st = reinterpret_cast<const T*>(h.store);
     const int64_t W = warps_global(), w = warp_id_global();
     // the block descriptor of the next task is loaded while this one runs, and
     // the task code of the one after it: a small task then costs one round trip
@@ -190,50 +250,13 @@ __device__ __noinline__ void pass_a(const Ops h, const double* __restrict__ D, i
         const int64_t code_nn = qnn < h.n_lr ? __ldg(h.lr_list + qnn) : 0;
         const BlkA bn = load_blk_a(h.blk + (code_n >> 8));
         const int kk0 = (int)(code & 255);
-        const int nrow = min(G, b.rank - kk0);
-        const T* row0 = st + b.off_a + (int64_t)kk0 * b.ns;
-        const double* xs = D + b.s0;
-        // each lane's products summed in T -- FP32 storage as an error-free
-        // (hi, lo) pair on the FP32 pipe -- then the warp's sums (warp_sums)
-        T hi[G][R], lo[G][R];
-#pragma unroll
-        for (int g = 0; g < G; ++g)
-#pragma unroll
-            for (int r = 0; r < R; ++r) { hi[g][r] = 0; lo[g][r] = 0; }
-        for (int64_t j0 = 0; j0 < b.ns; j0 += 32 * kUA) {
-            T v[kUA][G], xv[kUA][R];
-#pragma unroll
-            for (int u = 0; u < kUA; ++u) {
-                const int64_t j = j0 + u * 32 + lane;
-                const bool ok = j < b.ns;
-#pragma unroll
-                for (int g = 0; g < G; ++g) v[u][g] = (ok && g < nrow) ? __ldg(row0 + (int64_t)g * b.ns + j) : (T)0;
-#pragma unroll
-                for (int r = 0; r < R; ++r) xv[u][r] = ok ? (T)__ldcg(xs + (int64_t)r * N + j) : (T)0;
-            }
-#pragma unroll
-            for (int u = 0; u < kUA; ++u)
-#pragma unroll
-                for (int g = 0; g < G; ++g)
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const T pr = v[u][g] * xv[u][r];
-                        if constexpr (sizeof(T) == 4) {
-                            const T sum = hi[g][r] + pr, bp = sum - hi[g][r];
-                            lo[g][r] += (hi[g][r] - (sum - bp)) + (pr - bp);
-                            hi[g][r] = sum;
-                        } else {
-                            hi[g][r] += pr;
-                        }
-                    }
-        }
-        double tot[R];
-        warp_sums<T, G, R>(hi, lo, lane, tot);
-        constexpr int kSpan = 32 / G;   // lanes per row after the halving levels
-        const int g = lane / kSpan;
-        if (lane % kSpan == 0 && g < nrow) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) h.t[(b.toff + kk0 + g) * R + r] = tot[r];
+        if constexpr (R > 2) {
+            task_a<T, G, UA, R>(h, D, N, b, kk0);
+        } else {
+            const int lv = level_a(b.ns, R, sizeof(T));
+            if (lv == 0) task_a<T, G, UA, R>(h, D, N, b, kk0);
+            else if (lv == 1) task_a<T, G / 2, 2 * UA, R>(h, D, N, b, kk0);
+            else task_a<T, G / 4, 4 * UA, R>(h, D, N, b, kk0);
         }
         q = qn;
         code = code_n;

@@ -1653,12 +1653,12 @@ extern "C" int qdfn_set_hmatrix(qdfn_ctx* c, int64_t nb, const int64_t* range, c
         for (int64_t i = 0; i <= N; ++i) rowptr[(N + 1) + i] += base_n;
     }
     // warp tasks, largest first: pass A one per (low-rank block, group of
-    // rows_a rank rows) (cost ns x rows), pass B one per (block, 64-row slice)
+    // rows_a rank rows, fewer of long blocks) (cost ns x rows), pass B one per (block, 64-row slice)
     // (cost rows x inner size; a rank-0 block's task writes zero partials)
-    const int ga = Rk <= 2 ? hmat::rows_a<1>() : hmat::rows_a<4>();
     std::vector<std::pair<int64_t, int64_t>> ta, tb;   // (cost, code)
     for (int64_t q = 0; q < 2 * nb; ++q) {
         const hmat::Blk& B = blk[q];
+        const int ga = hmat::rows_a(Rk) >> hmat::level_a(B.ns, Rk, (int)esz);
         for (int64_t kk = 0; kk < B.rank; kk += ga)
             ta.push_back({B.ns * std::min<int64_t>(ga, B.rank - kk), (q << 8) | kk});
         const int64_t inner = B.rank < 0 ? B.ns : B.rank;
