@@ -8,7 +8,7 @@
 //                          consecutive receiver rows read consecutive words)
 //   low-rank  Vt, k x ns row-major, and U^T, k x nr
 // The product runs in two passes inside the persistent kernel, as WARP tasks
-// handed out in a fixed order over every warp of the grid (tree leaves hold at
+// dealt to the blocks and taken by their warps (tree leaves hold at
 // most `leaf` patches, so near-field blocks are small and a block per CTA
 // would leave most threads idle); pass B starts with the dense blocks, which
 // need nothing from pass A, and waits on a completion count of pass A (not on
@@ -32,7 +32,7 @@
 namespace qdfn {
 namespace hmat {
 
-struct Blk {   // 72 bytes
+struct Blk {   // (host) a block's place in the storage
     int64_t s0, ns, r0, nr;
     int64_t off_a;   // dense: D^T offset; low-rank: Vt offset
     int64_t off_b;   // low-rank: U^T offset
@@ -42,13 +42,25 @@ struct Blk {   // 72 bytes
     int32_t pad;
 };
 
+// A pass-A task: `rows` rank rows of a block, ns sources from s0 on
+struct alignas(16) TaskA {
+    int64_t off;     // first entry of the first row (rows ns apart)
+    int64_t t;       // its place in t (in units of R)
+    int32_t s0, ns, rows, pad;
+};
+// A pass-B task: up to 64 receiver rows of a block, K inner columns
+struct alignas(16) TaskB {
+    int64_t off;     // first row's entry of the first column (columns nr apart)
+    int64_t src;     // dense: first source; low-rank: first t (in units of R)
+    int64_t slot;    // first row's partial slot
+    int32_t nr, K, rows, pad;
+};
+
 struct Ops {
-    const Blk* blk;          // [2][nb]: shear blocks then normal blocks
-    int64_t nb;
     const void* store;       // element storage
-    const int64_t* lr_list;  // pass-A tasks: (blk index << 8) | first rank row of the group
+    const TaskA* lr_list;    // pass-A tasks
     int64_t n_lr;
-    const int64_t* tile_list;   // pass-B tasks: (blk index << 20) | 64-row slice; dense blocks' first
+    const TaskB* tile_list;  // pass-B tasks, dense blocks' first
     int64_t n_tiles;
     int64_t n_tiles_dense;      // the first n_tiles_dense tasks are dense blocks' (need no pass A)
     unsigned long long* a_done; // pass-A tasks completed since the launch began (monotone)
@@ -58,21 +70,34 @@ struct Ops {
     const int64_t* rowslot;  // slot indices
 };
 
-static_assert(sizeof(Blk) == 72 && alignof(Blk) == 8, "Blk is read as nine 8-byte words");
+static_assert(sizeof(TaskA) == 32 && sizeof(TaskB) == 48, "tasks are read as 16-byte words");
 
 constexpr int kSliceRows = 64;     // pass-B rows per warp task (two per lane)
-constexpr int kChunk = 1024;       // (shared-memory sizing of the H launches)
 constexpr int kMaxRank = 128;
 
-__device__ __forceinline__ int64_t warp_id_global() {
-    return (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-}
-__device__ __forceinline__ int64_t warps_global() { return (int64_t)gridDim.x * (blockDim.x >> 5); }
-// Task k of warp w among W warps: the lists are sorted largest first and dealt
-// out in snake order (rounds alternate direction), so that no warp takes the
+// Task k of block w among W: the lists are sorted largest first and dealt out to
+// the blocks in snake order (rounds alternate direction), so that none takes the
 // largest task of every round
 __device__ __forceinline__ int64_t snake_task(int64_t k, int64_t w, int64_t W) {
     return k * W + ((k & 1) ? W - 1 - w : w);
+}
+// A block's warps take its tasks from a counter in shared memory (ctr, zero at
+// the pass's start), one task ahead of the one they work on, whose record is
+// loaded meanwhile.  Dealt to the warps one by one, the slowest warp of a step had
+// 21 us of pass A where the average had 12.  6,000 triangles, us a step for the
+// two passes: 37 -> 26.5, FP64 107 -> 93, four instances 82 -> 57 (with the
+// descriptors in the task records, which saves each task a round trip).
+__device__ __forceinline__ int64_t claim_task(unsigned* ctr) {
+    unsigned n = 0;
+    if ((threadIdx.x & 31) == 0) n = atomicAdd(ctr, 1u);
+    return snake_task((int64_t)__shfl_sync(0xffffffffu, n, 0), blockIdx.x, gridDim.x);
+}
+template <class Task>
+__device__ __forceinline__ Task load_task(const Task* p) {
+    union { Task t; int4 w[sizeof(Task) / 16]; } u;
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(Task) / 16); ++k) u.w[k] = __ldg(reinterpret_cast<const int4*>(p) + k);
+    return u.t;
 }
 
 // rank rows per pass-A task of a short block: each lane keeps (hi, lo) sums for
@@ -90,20 +115,6 @@ __host__ __device__ constexpr int rounds_a(int R, int elem) { return elem == 4 &
 __host__ __device__ constexpr int level_a(int64_t ns, int R, int elem) {
     const int64_t batch = 32 * rounds_a(R, elem);
     return R > 2 || ns <= 2 * batch ? 0 : ns <= 8 * batch ? 1 : 2;
-}
-
-// A task's block descriptor, loaded once per task: nine independent 8-byte
-// loads (every lane the same words; the array's 72-byte stride keeps only
-// 8-byte alignment)
-__device__ __forceinline__ Blk load_blk(const Blk* p) {
-    const long long* w = reinterpret_cast<const long long*>(p);
-    Blk b;
-    b.s0 = __ldg(w); b.ns = __ldg(w + 1); b.r0 = __ldg(w + 2); b.nr = __ldg(w + 3);
-    b.off_a = __ldg(w + 4); b.off_b = __ldg(w + 5); b.toff = __ldg(w + 6); b.slot = __ldg(w + 7);
-    const int2 rk = __ldg(reinterpret_cast<const int2*>(w + 8));
-    b.rank = rk.x;
-    b.pad = rk.y;
-    return b;
 }
 
 // Warp sums of G values per lane (G = 1 to 8; R instances each) kept as FP32
@@ -159,26 +170,12 @@ __device__ __forceinline__ void warp_sums(T (&hi)[G][R], T (&lo)[G][R], int lane
     for (int r = 0; r < R; ++r) out[r] = sizeof(T) == 4 ? (double)hi[0][r] + (double)lo[0][r] : (double)hi[0][r];
 }
 
-// The fields of a block descriptor that pass A reads (five words).
-struct BlkA {
-    int64_t s0, ns, off_a, toff;
-    int rank;
-};
-__device__ __forceinline__ BlkA load_blk_a(const Blk* p) {
-    const long long* w = reinterpret_cast<const long long*>(p);
-    BlkA b;
-    b.s0 = __ldg(w); b.ns = __ldg(w + 1); b.off_a = __ldg(w + 4); b.toff = __ldg(w + 6);
-    b.rank = __ldg(reinterpret_cast<const int*>(w + 8));
-    return b;
-}
-
-// One pass-A task: up to G rank rows of block b from kk0 on, batches of UA 32-column
-// rounds
+// One pass-A task: up to G rank rows, batches of UA 32-column rounds
 template <class T, int G, int UA, int R>
-__device__ __forceinline__ void task_a(const Ops& h, const double* __restrict__ D, int64_t N, const BlkA& b, int kk0) {
+__device__ __forceinline__ void task_a(const Ops& h, const double* __restrict__ D, int64_t N, const TaskA& b) {
     const int lane = threadIdx.x & 31;
-    const int nrow = min(G, b.rank - kk0);
-    const T* row0 = reinterpret_cast<const T*>(h.store) + b.off_a + (int64_t)kk0 * b.ns;
+    const int nrow = b.rows;
+    const T* row0 = reinterpret_cast<const T*>(h.store) + b.off;
     const double* xs = D + b.s0;
     // each lane's products summed in T -- FP32 storage as an error-free
     // (hi, lo) pair on the FP32 pipe -- then the warp's sums (warp_sums)
@@ -187,11 +184,11 @@ __device__ __forceinline__ void task_a(const Ops& h, const double* __restrict__ 
     for (int g = 0; g < G; ++g)
 #pragma unroll
         for (int r = 0; r < R; ++r) { hi[g][r] = 0; lo[g][r] = 0; }
-    for (int64_t j0 = 0; j0 < b.ns; j0 += 32 * UA) {
+    for (int j0 = 0; j0 < b.ns; j0 += 32 * UA) {
         T v[UA][G], xv[UA][R];
 #pragma unroll
         for (int u = 0; u < UA; ++u) {
-            const int64_t j = j0 + u * 32 + lane;
+            const int j = j0 + u * 32 + lane;
             const bool ok = j < b.ns;
 #pragma unroll
             for (int g = 0; g < G; ++g) v[u][g] = (ok && g < nrow) ? __ldg(row0 + (int64_t)g * b.ns + j) : (T)0;
@@ -220,7 +217,7 @@ __device__ __forceinline__ void task_a(const Ops& h, const double* __restrict__ 
     const int g = lane / kSpan;
     if (lane % kSpan == 0 && g < nrow) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) h.t[(b.toff + kk0 + g) * R + r] = tot[r];
+        for (int r = 0; r < R; ++r) h.t[(b.t + g) * R + r] = tot[r];
     }
 }
 
@@ -232,35 +229,25 @@ __device__ __forceinline__ void task_a(const Ops& h, const double* __restrict__ 
 // B: beside the inlined solvers the loops lost registers and loads in flight
 // (6,000 triangles: the two passes 51 us a step, 42 out of line).
 template <class T, int R>
-__device__ __noinline__ void pass_a(const Ops h, const double* __restrict__ D, int64_t N, T*, double*) {
+__device__ __noinline__ void pass_a(const Ops h, const double* __restrict__ D, int64_t N, unsigned* ctr) {
     constexpr int G = rows_a(R), UA = rounds_a(R, sizeof(T));
     const int lane = threadIdx.x & 31;
-    const int64_t W = warps_global(), w = warp_id_global();
-    // the block descriptor of the next task is loaded while this one runs, and
-    // the task code of the one after it: a small task then costs one round trip
-    // (its data), not three (code, descriptor, data)
-    int64_t k = 0, q = snake_task(0, w, W);
-    const int64_t q1 = snake_task(1, w, W);
-    int64_t code = q < h.n_lr ? __ldg(h.lr_list + q) : 0;
-    int64_t code_n = q1 < h.n_lr ? __ldg(h.lr_list + q1) : 0;
-    BlkA b = load_blk_a(h.blk + (code >> 8));
+    if (h.n_lr <= 0) return;
+    int64_t q = claim_task(ctr);
+    TaskA b = load_task(h.lr_list + min(q, h.n_lr - 1));
     unsigned long long done = 0;
     while (q < h.n_lr) {
-        const int64_t qn = snake_task(++k, w, W), qnn = snake_task(k + 1, w, W);
-        const int64_t code_nn = qnn < h.n_lr ? __ldg(h.lr_list + qnn) : 0;
-        const BlkA bn = load_blk_a(h.blk + (code_n >> 8));
-        const int kk0 = (int)(code & 255);
+        const int64_t qn = claim_task(ctr);
+        const TaskA bn = load_task(h.lr_list + min(qn, h.n_lr - 1));
         if constexpr (R > 2) {
-            task_a<T, G, UA, R>(h, D, N, b, kk0);
+            task_a<T, G, UA, R>(h, D, N, b);
         } else {
             const int lv = level_a(b.ns, R, sizeof(T));
-            if (lv == 0) task_a<T, G, UA, R>(h, D, N, b, kk0);
-            else if (lv == 1) task_a<T, G / 2, 2 * UA, R>(h, D, N, b, kk0);
-            else task_a<T, G / 4, 4 * UA, R>(h, D, N, b, kk0);
+            if (lv == 0) task_a<T, G, UA, R>(h, D, N, b);
+            else if (lv == 1) task_a<T, G / 2, 2 * UA, R>(h, D, N, b);
+            else task_a<T, G / 4, 4 * UA, R>(h, D, N, b);
         }
         q = qn;
-        code = code_n;
-        code_n = code_nn;
         b = bn;
         ++done;
     }
@@ -280,46 +267,42 @@ __device__ __forceinline__ unsigned long long ld_acquire_ull(const unsigned long
 // (a lane per two rows).  The inner values (x of the block's sources, or t)
 // are held by the lanes and broadcast by shuffles; the matrix columns are
 // loaded sixteen at a time before they are used.  Tasks [lo, hi) of the list.
-template <class T, int R>
-__device__ void pass_b_range(const Ops& h, const double* __restrict__ D, int64_t N, int64_t lo, int64_t hi) {
+template <class T, int R, bool DENSE>
+__device__ __forceinline__ void pass_b_range(const Ops& h, const double* __restrict__ D, int64_t N, int64_t lo, int64_t hi,
+                             unsigned* ctr) {
     constexpr int U = sizeof(T) == 4 ? 16 : 8;   // columns loaded per batch: 2 x U loads per lane in flight
     const int lane = threadIdx.x & 31;
-    const T* st = reinterpret_cast<const T*>(h.store);
-    const int64_t W = warps_global(), w = warp_id_global();
     const int64_t n = hi - lo;
-    int64_t k = 0, q = snake_task(0, w, W);
-    int64_t code = q < n ? __ldg(h.tile_list + lo + q) : 0;
+    if (n <= 0) return;
+    int64_t q = claim_task(ctr);
+    TaskB b = load_task(h.tile_list + lo + min(q, n - 1));
     while (q < n) {
-        const Blk b = load_blk(h.blk + (code >> 20));
-        const int64_t i0 = (code & ((1 << 20) - 1)) * kSliceRows;
-        const int64_t qn = snake_task(++k, w, W);
-        const int64_t code_n = qn < n ? __ldg(h.tile_list + lo + qn) : 0;
-        const int64_t ia = i0 + lane, ib = i0 + 32 + lane;
-        const bool va = ia < b.nr, vb = ib < b.nr;
+        const int64_t qn = claim_task(ctr);
+        const TaskB bn = load_task(h.tile_list + lo + min(qn, n - 1));
+        const bool va = lane < b.rows, vb = 32 + lane < b.rows;
         T sa[R], sb[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) { sa[r] = 0; sb[r] = 0; }
-        const int64_t K = b.rank < 0 ? b.ns : b.rank;   // the inner dimension
-        const T* base = st + (b.rank < 0 ? b.off_a : b.off_b);
-        for (int64_t j0 = 0; j0 < K; j0 += 32) {
+        const int K = b.K;   // the inner dimension
+        const T* base = reinterpret_cast<const T*>(h.store) + b.off + lane;
+        for (int j0 = 0; j0 < K; j0 += 32) {
             T xv[R];
-            const int64_t jl = j0 + lane;
+            const int jl = j0 + lane;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 double v = 0.0;
-                if (jl < K)
-                    v = b.rank < 0 ? __ldcg(D + (int64_t)r * N + b.s0 + jl) : __ldcg(h.t + (b.toff + jl) * R + r);
+                if (jl < K) v = __ldcg(DENSE ? D + (int64_t)r * N + b.src + jl : h.t + (b.src + jl) * R + r);
                 xv[r] = (T)v;
             }
-            const int L = (int)min((int64_t)32, K - j0);
+            const int L = min(32, K - j0);
             for (int jb = 0; jb < L; jb += U) {
                 T ma[U], mb[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const bool ok = jb + u < L;
-                    const T* col = base + (j0 + jb + u) * b.nr;
-                    ma[u] = (ok && va) ? __ldg(col + ia) : (T)0;
-                    mb[u] = (ok && vb) ? __ldg(col + ib) : (T)0;
+                    const T* col = base + (int64_t)(j0 + jb + u) * b.nr;
+                    ma[u] = (ok && va) ? __ldg(col) : (T)0;
+                    mb[u] = (ok && vb) ? __ldg(col + 32) : (T)0;
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
@@ -334,12 +317,12 @@ __device__ void pass_b_range(const Ops& h, const double* __restrict__ D, int64_t
         }
         if (va)
 #pragma unroll
-            for (int r = 0; r < R; ++r) h.part[(b.slot + ia) * R + r] = (double)sa[r];
+            for (int r = 0; r < R; ++r) h.part[(b.slot + lane) * R + r] = (double)sa[r];
         if (vb)
 #pragma unroll
-            for (int r = 0; r < R; ++r) h.part[(b.slot + ib) * R + r] = (double)sb[r];
+            for (int r = 0; r < R; ++r) h.part[(b.slot + 32 + lane) * R + r] = (double)sb[r];
         q = qn;
-        code = code_n;
+        b = bn;
     }
 }
 
@@ -348,11 +331,11 @@ __device__ void pass_b_range(const Ops& h, const double* __restrict__ D, int64_t
 // bounded wait until a_done reaches a_target (every pass-A task of this step
 // has published its t), then the low-rank blocks' tasks.  a_target = 0: no
 // wait (pass A ran in an earlier launch).  Returns false if the wait gave up
-// (limit_ns, or another block's error in *gerr).
+// (limit_ns, or another block's error in *gerr).  ctr: the two parts' task counters.
 template <class T, int R>
 __device__ __noinline__ bool pass_b(const Ops h, const double* __restrict__ D, int64_t N, unsigned long long a_target,
-                       uint64_t limit_ns, const int* gerr) {
-    pass_b_range<T, R>(h, D, N, 0, h.n_tiles_dense);
+                       uint64_t limit_ns, const int* gerr, unsigned* ctr) {
+    pass_b_range<T, R, true>(h, D, N, 0, h.n_tiles_dense, ctr);
     if (h.n_tiles <= h.n_tiles_dense) return true;
     int ok = 1;
     if (a_target > 0 && (threadIdx.x & 31) == 0 && ld_acquire_ull(h.a_done) < a_target) {
@@ -367,7 +350,7 @@ __device__ __noinline__ bool pass_b(const Ops h, const double* __restrict__ D, i
     }
     ok = __shfl_sync(0xffffffffu, ok, 0);
     if (!ok) return false;
-    pass_b_range<T, R>(h, D, N, h.n_tiles_dense, h.n_tiles);
+    pass_b_range<T, R, false>(h, D, N, h.n_tiles_dense, h.n_tiles, ctr + 1);
     return true;
 }
 

@@ -226,7 +226,7 @@ int configure_launch(qdfn_ctx* c) {
     if (const char* e = std::getenv("QDFN_PAIR_SOLVE")) c->pair_solve = std::max(0, std::min(2, std::atoi(e)));
     int64_t want_blocks;
     if (c->hmat) {
-        c->smem = (size_t)Rk * hmat::kChunk * xsz + (size_t)hmat::kMaxRank * Rk * sizeof(double);
+        c->smem = 0;
         c->nchunk = c->nchunk2 = 0;
         c->chunk_len = c->chunk_len2 = c->rb_small0 = 0;
         want_blocks = (std::max<int64_t>(c->hops.n_tiles, c->hops.n_lr) + kSimThreads / 32 - 1) / (kSimThreads / 32);
@@ -1678,16 +1678,29 @@ extern "C" int qdfn_set_hmatrix(qdfn_ctx* c, int64_t nb, const int64_t* range, c
         tb.begin(), tb.end(), [&](const std::pair<int64_t, int64_t>& x) { return blk[x.second >> 20].rank < 0; });
     std::sort(tb.begin(), tb.begin() + n_dense, by_cost);
     std::sort(tb.begin() + n_dense, tb.end(), by_cost);
-    std::vector<int64_t> lr, tiles;
-    for (auto& x : ta) lr.push_back(x.second);
-    for (auto& x : tb) tiles.push_back(x.second);
+    std::vector<hmat::TaskA> lr;
+    std::vector<hmat::TaskB> tiles;
+    for (auto& x : ta) {
+        const hmat::Blk& B = blk[x.second >> 8];
+        const int64_t kk = x.second & 255;
+        const int64_t ga = hmat::rows_a(Rk) >> hmat::level_a(B.ns, Rk, (int)esz);
+        lr.push_back({B.off_a + kk * B.ns, B.toff + kk, (int32_t)B.s0, (int32_t)B.ns,
+                      (int32_t)std::min<int64_t>(ga, B.rank - kk), 0});
+    }
+    for (auto& x : tb) {
+        const hmat::Blk& B = blk[x.second >> 20];
+        const int64_t i0 = (x.second & ((1 << 20) - 1)) * hmat::kSliceRows;
+        const bool dense = B.rank < 0;
+        tiles.push_back({(dense ? B.off_a : B.off_b) + i0, dense ? B.s0 : B.toff, B.slot + i0, (int32_t)B.nr,
+                         (int32_t)(dense ? B.ns : B.rank), (int32_t)std::min<int64_t>(hmat::kSliceRows, B.nr - i0), 0});
+    }
     // device copies
     release_hmat(c);
     c->release(c->E); c->release(c->Kn);
     c->E = c->Kn = nullptr;
     int rc;
-    hmat::Blk* dblk; unsigned char* dstore; int64_t *dlr, *dtiles, *drp, *drs; double *dt, *dpart;
-    if ((rc = dcopy(c, blk.data(), blk.size(), &dblk)) || (rc = dcopy(c, hbuf.data(), hbuf.size(), &dstore)) ||
+    unsigned char* dstore; hmat::TaskA* dlr; hmat::TaskB* dtiles; int64_t *drp, *drs; double *dt, *dpart;
+    if ((rc = dcopy(c, hbuf.data(), hbuf.size(), &dstore)) ||
         (rc = dcopy(c, lr.data(), lr.size(), &dlr)) || (rc = dcopy(c, tiles.data(), tiles.size(), &dtiles)) ||
         (rc = dcopy(c, rowptr.data(), rowptr.size(), &drp)) ||
         (rc = dcopy(c, rowslot.data(), rowslot.size(), &drs)))
@@ -1697,7 +1710,7 @@ extern "C" int qdfn_set_hmatrix(qdfn_ctx* c, int64_t nb, const int64_t* range, c
     if ((rc = c->dalloc(&dpart, (size_t)std::max<int64_t>(slot, 1) * Rk))) return rc;
     c->hbufs.push_back(dpart);
     hmat::Ops& h = c->hops;
-    h.blk = dblk; h.nb = nb; h.store = dstore; h.lr_list = dlr; h.n_lr = (int64_t)lr.size();
+    h.store = dstore; h.lr_list = dlr; h.n_lr = (int64_t)lr.size();
     h.tile_list = dtiles; h.n_tiles = (int64_t)tiles.size(); h.t = dt; h.part = dpart;
     h.n_tiles_dense = n_dense;
     h.a_done = c->tile_ctr;   // reset in every launch's prologue

@@ -1081,10 +1081,9 @@ template <class M, int R, bool HM>
 __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, const int blk) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     using X = typename M::X;
-    // dense: [stage ring | mbarriers, stage descriptors | two x buffers];
-    // H-matrix: [x | rank accumulators]
-    X* xs = reinterpret_cast<X*>(HM ? smem_raw : smem_raw + kPipeBytes + kMbarBytes);
-    double* hacc = reinterpret_cast<double*>(smem_raw + (size_t)R * hmat::kChunk * sizeof(X));
+    // dense: [stage ring | mbarriers, stage descriptors | two x buffers]
+    X* xs = reinterpret_cast<X*>(smem_raw + kPipeBytes + kMbarBytes);
+    __shared__ unsigned s_htask[3];   // H-matrix: the passes' task counters
     Pipe pipe;
     if constexpr (!HM) pipe_init(pipe, smem_raw);
     // s_dt: Dt of the current step; s_dtn: the next step's, decided with the
@@ -1286,6 +1285,7 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
         const bool pre = it > 0 && s_next_valid == it;
         if (use_order && !pre && threadIdx.x < 32) rb_order(p, cpar, s_order[it & 1]);
         if (threadIdx.x >= 32 && threadIdx.x < 32 + R) pass_scalars(threadIdx.x - 32);
+        if (HM && threadIdx.x < 3) s_htask[threadIdx.x] = 0;
         red_init();
         __syncthreads();
         const X* xdc = reinterpret_cast<const X*>(p.xd) + (size_t)par * p.xd_stride;
@@ -1458,10 +1458,10 @@ __device__ __forceinline__ void sim_run(const SimParams& p, int64_t nsteps, cons
         // ---------------------------------------------------------- P2
         if constexpr (HM) {
             const double* Dcur = par ? p.Dn : p.D;
-            hmat::pass_a<X, R>(p.h, Dcur, N, xs, hacc);
+            hmat::pass_a<X, R>(p.h, Dcur, N, s_htask);
             // pass B's low-rank tasks wait for this step's pass-A count, not a grid barrier
             if (!hmat::pass_b<X, R>(p.h, Dcur, N, (unsigned long long)(it + 1) * (unsigned long long)p.h.n_lr,
-                                    kWaitLimitNs, p.gerr))
+                                    kWaitLimitNs, p.gerr, s_htask + 1))
                 atomicExch(p.gerr, QDFN_ERR_TIMEOUT);
             if (!grid_barrier(p, deadline)) return;
         } else if constexpr (sizeof(X) == 8) {
@@ -1955,14 +1955,17 @@ __global__ void __launch_bounds__(kSimThreads, 1) k_apply(SimParams p) {
 
 template <class X, int R>
 __global__ void __launch_bounds__(kSimThreads, 1) k_hmat_a(SimParams p) {
-    extern __shared__ unsigned char smem_raw[];
-    hmat::pass_a<X, R>(p.h, p.D, p.N, reinterpret_cast<X*>(smem_raw),
-                       reinterpret_cast<double*>(smem_raw + (size_t)R * hmat::kChunk * sizeof(X)));
+    __shared__ unsigned s_task;
+    if (threadIdx.x == 0) s_task = 0;
+    __syncthreads();
+    hmat::pass_a<X, R>(p.h, p.D, p.N, &s_task);
 }
 template <class X, int R>
 __global__ void __launch_bounds__(kSimThreads, 1) k_hmat_b(SimParams p) {
-    extern __shared__ unsigned char smem_raw[];
-    hmat::pass_b<X, R>(p.h, p.D, p.N, 0ull, kWaitLimitNs, p.gerr);   // pass A ran in the launch before
+    __shared__ unsigned s_task[2];
+    if (threadIdx.x < 2) s_task[threadIdx.x] = 0;
+    __syncthreads();
+    hmat::pass_b<X, R>(p.h, p.D, p.N, 0ull, kWaitLimitNs, p.gerr, s_task);   // pass A ran in the launch before
 }
 // receiver-row sums of the operator-only H product: 32 rows per 256-thread
 // block (eight threads per row: four per matrix)
