@@ -353,39 +353,39 @@ extern "C" int qdfn_ctx_create(qdfn_ctx** out, const qdfn_problem* pr) {
     c->eta = pr->G / 2 / std::sqrt(pr->G / pr->rho);
     const int Rk = kernel_R(c->R);
     const size_t RN = (size_t)Rk * N;
-    int rc = 0;
-#define A(ptr, n) if (!rc) rc = c->dalloc(&c->ptr, n)
+    // the context's arrays in one zeroed allocation, those with initial values first
+    // and filled by one copy: an allocation, a memset and a copy for each cost 0.5 ms
+    // of a short run's host time (200 steps of 800 patches through `main` 7.4 -> 6.9 ms)
+    struct Part { void** ptr; size_t off; };
+    std::vector<Part> parts;
+    size_t arena = 0;
+    auto part = [&](auto** ptr, size_t n) {
+        parts.push_back({reinterpret_cast<void**>(ptr), arena});
+        arena += (n * sizeof(**ptr) + 16 + 255) / 256 * 256;   // (16 bytes past the end may be read)
+    };
+#define A(ptr, n) part(&c->ptr, n)
     A(a, RN); A(b, RN); A(Dc, RN); A(F0, RN); A(tau0, RN); A(sigma0, RN); A(Vconst, RN);
     A(ra, RN); A(rDc, RN);
-    A(mass, RN); A(omega, RN); A(kself, (size_t)N); A(unstable, RN); A(has_unstable, (size_t)Rk);
-    A(la, RN); A(lth0, RN); A(dref, 2 * (size_t)Rk);
+    A(mass, RN); A(unstable, RN); A(has_unstable, (size_t)Rk);
+    A(la, RN); A(lth0, RN);
     // the six host-visible state fields in one block, in the order of the
     // state-transfer calls, so that contiguous host buffers move in one copy
     double* state6 = nullptr;
-    if (!rc) rc = c->dalloc(&state6, 6 * RN);
-    if (!rc) {
-        c->V = state6; c->D = state6 + RN; c->theta = state6 + 2 * RN;
-        c->fric = state6 + 3 * RN; c->accel = state6 + 4 * RN; c->sig_old = state6 + 5 * RN;
-    }
+    part(&state6, 6 * RN);
+    double* Tdt = nullptr;           // T and dt side by side, for the same reason
+    part(&Tdt, 2 * (size_t)Rk);
+    A(step, (size_t)Rk); A(nrec, (size_t)Rk); A(status, (size_t)Rk);
+    const size_t filled = arena;     // (the rest starts as zeros)
+    A(omega, RN); A(kself, (size_t)N); A(dref, 2 * (size_t)Rk);
     A(Vn, RN); A(Dn, RN); A(thn, RN); A(fn, RN); A(sn, RN); A(dtall, RN); A(tld, RN); A(knd, RN);
     A(instab, RN); A(flag, RN); A(sw, RN); A(sw_n, RN); A(accel_n, RN);
-    double* Tdt = nullptr;           // T and dt side by side, for the same reason
-    if (!rc) rc = c->dalloc(&Tdt, 2 * (size_t)Rk);
-    if (!rc) { c->T = Tdt; c->dt = Tdt + Rk; }
-    A(step, (size_t)Rk); A(nrec, (size_t)Rk); A(status, (size_t)Rk);
     const size_t hr = (size_t)Rk * std::max<int64_t>(pr->max_records, 1);
     A(hT, hr); A(hDt, hr); A(hV, hr * N); A(hD, hr * N); A(hth, hr * N); A(hs, hr * N);
     // launch control words side by side: [0] error flag, [1] barrier arrivals,
     // [2] barrier generation, and from the second line the reductions' words --
     // all cleared by one memset per launch
     int* ctrl = nullptr;
-    if (!rc) rc = c->dalloc(&ctrl, kCtrlBytes / sizeof(int));
-    if (!rc) {
-        c->gerr = ctrl;
-        c->bar_count = reinterpret_cast<unsigned*>(ctrl + 1);
-        c->bar_gen = reinterpret_cast<unsigned*>(ctrl + 2);
-        c->red = reinterpret_cast<unsigned long long*>(ctrl + 32);
-    }
+    part(&ctrl, kCtrlBytes / sizeof(int));
     A(prof, kCounters); A(tile_ctr, kSets); A(spec_ctr, kSets);
     // per-step counters, kSets sets used by steps in turn (a step uses one, streams
     // ahead into the next, and resets the one two ahead)
@@ -393,10 +393,20 @@ extern "C" int qdfn_ctx_create(qdfn_ctx** out, const qdfn_problem* pr) {
     A(solve_ctr, kSets); A(tmax, 4 * kSets); A(rb_done, kSets * (size_t)c->rb_stride);
     A(rb_solved, kSets * (size_t)c->rb_stride); A(rb_hot, kSets * (size_t)c->rb_stride);
 #undef A
+    unsigned char* base = nullptr;
+    int rc = c->dalloc(&base, arena);
     if (rc) { delete c; return rc; }
+    for (const Part& q : parts) *q.ptr = base + q.off;
+    c->V = state6; c->D = state6 + RN; c->theta = state6 + 2 * RN;
+    c->fric = state6 + 3 * RN; c->accel = state6 + 4 * RN; c->sig_old = state6 + 5 * RN;
+    c->T = Tdt; c->dt = Tdt + Rk;
+    c->gerr = ctrl;
+    c->bar_count = reinterpret_cast<unsigned*>(ctrl + 1);
+    c->bar_gen = reinterpret_cast<unsigned*>(ctrl + 2);
+    c->red = reinterpret_cast<unsigned long long*>(ctrl + 32);
     // host-side initialisation (Main_D :41-131): padded instances replicate instance 0
     std::vector<double> ha(RN), hb(RN), hDc(RN), hF0(RN), htau0(RN), hs0(RN), hVc(RN), hm(RN),
-        hth(RN), hV(RN), hf(RN), hzero(RN, 0.0);
+        hth(RN), hV(RN), hf(RN);
     std::vector<unsigned char> hun(RN);
     std::vector<double> hla(RN), hlth(RN);
     std::vector<int> hhas(Rk, 0);
@@ -424,22 +434,20 @@ extern "C" int qdfn_ctx_create(qdfn_ctx** out, const qdfn_problem* pr) {
     // correctly rounded here as on the device
     std::vector<double> hra(RN), hrDc(RN);
     for (size_t q = 0; q < RN; ++q) { hra[q] = 1.0 / ha[q]; hrDc[q] = 1.0 / hDc[q]; }
-    std::vector<double> ones(Rk, 1.0), zeros(Rk, 0.0);
-    std::vector<int64_t> z64(Rk, 0);
-    std::vector<int> z32(Rk, 0);
-    if ((rc = h2d(c->a, ha.data(), RN * 8)) || (rc = h2d(c->b, hb.data(), RN * 8)) ||
-        (rc = h2d(c->ra, hra.data(), RN * 8)) || (rc = h2d(c->rDc, hrDc.data(), RN * 8)) ||
-        (rc = h2d(c->Dc, hDc.data(), RN * 8)) || (rc = h2d(c->F0, hF0.data(), RN * 8)) ||
-        (rc = h2d(c->tau0, htau0.data(), RN * 8)) || (rc = h2d(c->sigma0, hs0.data(), RN * 8)) ||
-        (rc = h2d(c->Vconst, hVc.data(), RN * 8)) || (rc = h2d(c->mass, hm.data(), RN * 8)) ||
-        (rc = h2d(c->unstable, hun.data(), RN)) || (rc = h2d(c->has_unstable, hhas.data(), Rk * 4)) ||
-        (rc = h2d(c->V, hV.data(), RN * 8)) || (rc = h2d(c->theta, hth.data(), RN * 8)) ||
-        (rc = h2d(c->fric, hf.data(), RN * 8)) || (rc = h2d(c->sig_old, hs0.data(), RN * 8)) ||
-        (rc = h2d(c->D, hzero.data(), RN * 8)) || (rc = h2d(c->accel, hzero.data(), RN * 8)) ||
-        (rc = h2d(c->T, zeros.data(), Rk * 8)) || (rc = h2d(c->dt, ones.data(), Rk * 8)) ||
-        (rc = h2d(c->step, z64.data(), Rk * 8)) || (rc = h2d(c->nrec, z64.data(), Rk * 8)) ||
-        (rc = h2d(c->status, z32.data(), Rk * 4)) || (rc = h2d(c->la, hla.data(), RN * 8)) ||
-        (rc = h2d(c->lth0, hlth.data(), RN * 8))) {
+    const std::vector<double> ones(Rk, 1.0);
+    std::vector<unsigned char> image(filled, 0);   // (D, accel, T, step, nrec and status start as zeros)
+    auto put = [&](void* dst, const void* src, size_t bytes) {
+        std::memcpy(image.data() + (static_cast<unsigned char*>(dst) - base), src, bytes);
+    };
+    put(c->a, ha.data(), RN * 8); put(c->b, hb.data(), RN * 8); put(c->Dc, hDc.data(), RN * 8);
+    put(c->ra, hra.data(), RN * 8); put(c->rDc, hrDc.data(), RN * 8); put(c->F0, hF0.data(), RN * 8);
+    put(c->tau0, htau0.data(), RN * 8); put(c->sigma0, hs0.data(), RN * 8); put(c->Vconst, hVc.data(), RN * 8);
+    put(c->mass, hm.data(), RN * 8); put(c->unstable, hun.data(), RN); put(c->has_unstable, hhas.data(), Rk * 4);
+    put(c->la, hla.data(), RN * 8); put(c->lth0, hlth.data(), RN * 8);
+    put(c->V, hV.data(), RN * 8); put(c->theta, hth.data(), RN * 8); put(c->fric, hf.data(), RN * 8);
+    put(c->sig_old, hs0.data(), RN * 8);
+    put(c->dt, ones.data(), Rk * 8);
+    if ((rc = h2d(base, image.data(), filled))) {
         delete c;
         return rc;
     }
