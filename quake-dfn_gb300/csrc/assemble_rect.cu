@@ -31,8 +31,8 @@ __device__ __noinline__ void general_gradients(double alpha, double dip, double 
 // time: what depends on the source alone (sines and cosines, the medium) is
 // formed once per block and turn, what depends on the receiver alone once per
 // turn.  Bound by the FP64 pipe.  Against one pair per thread and turn with all
-// of okada.cuh: 5,850 x 5,850 patches 473.6 -> 88.4 ms, 800 x 800 9.80 -> 1.88
-// ms, 61 x 64 (122 warps: the length of one pair's chain) 252 -> 65 us.
+// of okada.cuh: 5,850 x 5,850 patches 473.6 -> 86.6 ms, 800 x 800 9.80 -> 1.84
+// ms, 61 x 64 (122 warps: the length of one pair's chain) 252 -> 64 us.
 __global__ void __launch_bounds__(kAsmThreads)
 k_assemble_rect(int64_t n_src, const double* __restrict__ src, int64_t n_recv,
                 const double* __restrict__ recv, double G, double nu, double* __restrict__ Ks,

@@ -23,9 +23,11 @@
 // R is formed as okada.cuh forms it, to the last bit but for rare ties, and so
 // are R + xi and R + eta, whose cancellation dominates the rounding error of
 // both; the zeroing of |xi|, |eta|, |q| < 1e-6 inside R, Y~ and D~ alone is
-// kept.  Where R + xi, R + eta or R + D~ is below 1e-9 R, or anything is not
+// kept.  Where R + xi, R + eta or R + D~ is below 2^-30 R, or anything is not
 // finite, corner_sums() reports it and the caller evaluates okada.cuh.
 #pragma once
+#include <cstring>
+
 #include "okada.cuh"
 
 namespace qdfn {
@@ -63,8 +65,26 @@ QDFN_HD void root(double R2, double& R, double& i1) {
     const double r = R2 * i1;
     R = fma(fma(-r, r, R2), 0.5 * i1, r);
 }
-// DCCON2's EPS rule
-QDFN_HD double zero_small(double v) { return fabs(v) < 1.0e-6 ? 0.0 : v; }
+QDFN_HD long long dbits(double v) {
+#ifdef __CUDA_ARCH__
+    return __double_as_longlong(v);
+#else
+    long long b;
+    memcpy(&b, &v, 8);
+    return b;
+#endif
+}
+// DCCON2's EPS rule, |v| < 1e-6 (compared as integers, like the checks below: an
+// FP64 comparison takes the FP64 pipe)
+QDFN_HD double zero_small(double v) {
+    return (dbits(v) & 0x7fffffffffffffffll) < 0x3eb0c6f7a0b5ed8dll ? 0.0 : v;
+}
+QDFN_HD int hi_word(double v) { return (int)(dbits(v) >> 32); }
+// x > 2^-30 R (R >= 0; x NaN passes, R is checked)
+QDFN_HD bool well_above(double x, int hiR) {
+    const int h = hi_word(x);
+    return h > 0 && h > hiR - (30 << 20);
+}
 
 // Corner functions, and differences of them over xi
 struct Corner {
@@ -81,8 +101,8 @@ QDFN_HD Corner corner(double XI, double x, double ET, double e, double q2, doubl
     double R;
     root(R2, R, c.i1);
     const double RX = R + x, RE = R + e;
-    const double tiny = 1e-9 * R;
-    ok = ok && RX > tiny && RE > tiny && R < 1e30;
+    const int hiR = hi_word(R);
+    ok = ok && well_above(RX, hiR) && well_above(RE, hiR) && (unsigned)hiR < 0x46293e59u;   // R < 1e30
     const double i2 = c.i1 * c.i1;
     c.i3 = i2 * c.i1;
     c.Xi3 = XI * c.i3;
@@ -98,7 +118,7 @@ QDFN_HD Corner corner(double XI, double x, double ET, double e, double q2, doubl
     c.XxxY32 = XI * c.xxY32;
     if constexpr (IMG) {
         const double RD = R + D;
-        ok = ok && RD > tiny;
+        ok = ok && well_above(RD, hiR);
         const double iRD = recip1(RD);
         c.i5 = c.i3 * i2;
         c.Xi5 = XI * c.i5;
