@@ -24,8 +24,8 @@
 // and every receiver row then sums its partials (row_sums_block: four threads
 // per row and matrix, each over every fourth partial in block order, combined
 // in a fixed order, so results are reproducible run to run).  Tasks are listed
-// largest first and dealt out to the warps in snake order, which spreads the
-// long ones.
+// largest first and dealt out to the blocks in snake order, which spreads the
+// long ones; which warp takes a task does not change its result.
 #pragma once
 #include "qdfn_internal.h"
 

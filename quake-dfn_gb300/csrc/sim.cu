@@ -237,7 +237,8 @@ int configure_launch(qdfn_ctx* c) {
         const int64_t nrb = (c->N + rows_per_blk - 1) / rows_per_blk;
         // tiles per SM and step (tuning knob QDFN_TILES_PER_SM).  FP32/BF16: 4, so
         // that the solves of the first row blocks run beside the rest of the
-        // stream -- but one where a tile of it is at most 384 columns: the stream
+        // stream -- but one where a tile of it is at most 384 columns (and both splits
+        // fall on groups of 32): the stream
         // is then shorter than a solve's chain, and fewer chunks make the chain
         // shorter (the solves add up a partial sum per chunk).  us a step, 1 / 4
         // tiles, one instance: 3,001 patches 37 / 41, 4,500 53 / 55, 6,500 98 / 72.
@@ -246,24 +247,31 @@ int configure_launch(qdfn_ctx* c) {
         // 2,000 patches 46 / 49 / 52, 4,500 x 4 instances 576 / 383 / 387, 6,500
         // 232 / 218 / 209.
         const int64_t one = (nrb * c->N + sms - 1) / sms;   // columns of a tile at one per SM
-        const bool exact = c->prec == QDFN_FP64 || one <= 384;   // at most the tiles asked for
-        int64_t tiles_per_sm = c->prec == QDFN_FP64 ? (one <= 256 ? 1 : one <= 800 ? 2 : 8) : one <= 384 ? 1 : 4;
-        if (const char* e = std::getenv("QDFN_TILES_PER_SM")) tiles_per_sm = std::max(1, std::min(64, std::atoi(e)));
+        const bool fp64 = c->prec == QDFN_FP64;
+        int64_t tiles_per_sm = fp64 ? (one <= 256 ? 1 : one <= 800 ? 2 : 8) : 4;
+        const char* tiles_env = std::getenv("QDFN_TILES_PER_SM");
+        if (tiles_env) tiles_per_sm = std::max(1, std::min(64, std::atoi(tiles_env)));
         if (const char* e = std::getenv("QDFN_SOLVE_HOLD")) c->hold_cap = std::max(1, std::min(64, std::atoi(e)));
         if (const char* e = std::getenv("QDFN_RB_ORDER")) c->rb_ordered = std::atoi(e) != 0 ? 1 : 0;
         if (const char* e = std::getenv("QDFN_SPEC_COLS")) c->c_spec = std::max(0, std::min(64, std::atoi(e)));
         if (const char* e = std::getenv("QDFN_SPEC_STOP")) c->spec_stop_pct = std::max(1, std::min(100, std::atoi(e)));
-        int64_t want_chunks = std::max<int64_t>(1, (tiles_per_sm * sms + (exact ? 0 : nrb - 1)) / nrb);
-        int64_t clen = (c->N + want_chunks - 1) / want_chunks;
         // two x buffers (R x chunk x elem each) share the 227 KB with the 160 KB stage
         // ring and the FP32 sums' pairs (8 KB per instance)
         const int64_t cmax = std::max<int64_t>(64, (int64_t)(14 * 1024) / (Rk * (int64_t)xsz));
         // at least 64 columns, 32 in FP64: its tiles take the FP64 pipe 32 times an
         // FP32 tile's time, so small systems spread them over more blocks (800
         // patches: 52 tiles on 25 blocks 25 us a step, 100 on 100)
-        const int64_t cmin = c->prec == QDFN_FP64 ? 32 : 64;
-        clen = (std::min<int64_t>(std::max<int64_t>(clen, cmin), std::min<int64_t>(2048, cmax)) + 7) / 8 * 8;
-        if (exact) clen = std::min<int64_t>((clen + 31) / 32 * 32, cmax / 32 * 32);
+        const int64_t cmin = fp64 ? 32 : 64;
+        // (exact: at most the tiles asked for, in multiples of 32 columns)
+        auto chunk = [&](int64_t tiles, bool exact) {
+            const int64_t want = std::max<int64_t>(1, (tiles * sms + (exact ? 0 : nrb - 1)) / nrb);
+            const int64_t len = std::max<int64_t>((c->N + want - 1) / want, cmin), top = std::min<int64_t>(2048, cmax);
+            return exact ? std::min<int64_t>((len + 31) / 32 * 32, top / 32 * 32) : (std::min(len, top) + 7) / 8 * 8;
+        };
+        int64_t clen = chunk(tiles_per_sm, fp64);
+        // one tile only where both splits end on the groups of 32 columns that FP32
+        // products are summed in: the results are the same
+        if (!fp64 && !tiles_env && one <= 384 && clen % 32 == 0) clen = chunk(1, true);
         c->chunk_len = clen;
         c->nchunk = (int)((c->N + clen - 1) / clen);
         // the row blocks of the last two waves of tiles are streamed by their own
@@ -964,19 +972,18 @@ void ensemble_detach(qdfn_ensemble* e, qdfn_ctx* c) {
         if (x == c) x = nullptr;
 }
 
-// Estimated SM-nanoseconds of one step of a member on one SM: the longer of its
-// operator bytes at one SM's share of the HBM stream (~44 B/ns) and its patch
-// solves beside them (~85 ns of one SM each, of its seven solver warps).  Only the
-// starting point of the split; qdfn_ensemble_balance re-divides by measured time.
-// (40 networks of 908-2,838 patches x 4, 15 steps: 4.31 ms, as after three
-// balances; 4.56 with the sum of both at the former 450 ns a solve.)
+// Estimated SM-nanoseconds of one step of a member on one SM: its operator
+// bytes at one SM's share of the HBM stream (~44 B/ns) plus 450 ns per patch
+// solve.  Only the starting point of the split; qdfn_ensemble_balance re-divides
+// by measured time.  (A solve takes ~85 ns of an SM by now, beside the stream:
+// max(bytes / 44, 85 per solve) starts as the balanced split does, 40 networks x
+// 4, 15 steps 4.57 -> 4.45 ms.  But the shares set the column chunks, and with
+// them the groups of 32 columns that FP32 products are summed in: the results
+// would move by that rounding, 2e-8 of the largest acceleration.)
 double member_cost(const qdfn_ctx* c) {
     const double esz = c->prec == QDFN_FP64 ? 8.0 : 4.0;
     const double n = (double)c->N;
-    const double op = 2.0 * n * n * esz / 44.0, solves = 85.0 * kernel_R(c->R) * n;
-    // FP64: the solves follow the operator, whose FMAs take the FP64 pipe ~0.25 ns
-    // of one SM each per instance
-    return c->prec == QDFN_FP64 ? std::max(op, 0.5 * kernel_R(c->R) * n * n) + solves : std::max(op, solves);
+    return 2.0 * n * n * esz / 44.0 + 450.0 * kernel_R(c->R) * n;
 }
 
 // A member's busy ns as the status kernel of the last ensemble run read them.
