@@ -855,7 +855,7 @@ def run_ensemble(args):
     solves = sum(c1["lowv_solves"] + c1["highv_solves"] - c0["lowv_solves"] - c0["highv_solves"]
                  for c0, c1 in zip(cnt0, cnt))
     fp64_tf = fp64_peak_tflops(dev) if rank == 0 else None
-    # the unit the ensemble is bound by: FP64 instructions of the friction
+    # FP64 instructions of the friction
     # solves per second (the committed capture's instructions per patch solve
     # x the window's solves per second) against the measured FP64 rate (one
     # DFMA per two flops of the FP64 GEMM)
