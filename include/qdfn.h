@@ -409,6 +409,12 @@ int qdfn_apply_dense_noalloc(int64_t N, const double* Ks, const double* Kn, int6
  * division.  No counterpart in the reference (Julia's `/`). */
 int qdfn_check_division(int64_t n, const double* x, const double* d, double* q, void* stream);
 
+/* qdfn_assemble_rect_dev with every pair by the published formulas term by term
+ * (scripts/Functions_OKADA3D.jl), where the assembly sums corner functions:
+ * slower by a factor of five, and what its entries are compared with. */
+int qdfn_check_rect(int64_t n_src, const double* src, int64_t n_recv, const double* recv, double G, double nu,
+                    double* Ks, double* Kn, int64_t ld, int layout, void* stream);
+
 /* ---- input parsing and discretisation (host only) ------------------------ */
 /* The reference's RUN2 front end, so a caller goes from the bulk text file to
  * the segment table without Julia.  Tables are row-major doubles.  Two-call

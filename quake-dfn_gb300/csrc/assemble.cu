@@ -42,16 +42,27 @@ struct DevBuf {
 
 using namespace qdfn;
 
-extern "C" int qdfn_assemble_rect_dev(int64_t n_src, const double* src, int64_t n_recv,
-                                      const double* recv, double G, double nu, double* Ks,
-                                      double* Kn, int64_t ld, int layout, void* stream) {
+static int assemble_rect_dev(int64_t n_src, const double* src, int64_t n_recv, const double* recv, double G, double nu,
+                             double* Ks, double* Kn, int64_t ld, int layout, void* stream, bool general) {
     int rc = check_common(n_src, n_recv, ld, layout);
     if (rc) return rc;
     if (n_src == 0 || n_recv == 0) return QDFN_OK;
     if (!src || !recv || !Ks || !Kn) return fail(QDFN_ERR_INVALID, "null pointer");
-    launch_assemble_rect((cudaStream_t)stream, n_src, src, n_recv, recv, G, nu, Ks, Kn, ld, layout);
+    launch_assemble_rect((cudaStream_t)stream, n_src, src, n_recv, recv, G, nu, Ks, Kn, ld, layout,
+                         general);
     QDFN_CUDA(cudaGetLastError());
     return QDFN_OK;
+}
+
+extern "C" int qdfn_assemble_rect_dev(int64_t n_src, const double* src, int64_t n_recv,
+                                      const double* recv, double G, double nu, double* Ks,
+                                      double* Kn, int64_t ld, int layout, void* stream) {
+    return assemble_rect_dev(n_src, src, n_recv, recv, G, nu, Ks, Kn, ld, layout, stream, false);
+}
+
+extern "C" int qdfn_check_rect(int64_t n_src, const double* src, int64_t n_recv, const double* recv, double G,
+                               double nu, double* Ks, double* Kn, int64_t ld, int layout, void* stream) {
+    return assemble_rect_dev(n_src, src, n_recv, recv, G, nu, Ks, Kn, ld, layout, stream, true);
 }
 
 extern "C" int qdfn_assemble_rect(int64_t n_src, const double* src, int64_t n_recv,

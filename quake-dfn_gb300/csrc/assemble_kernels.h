@@ -6,8 +6,9 @@
 
 namespace qdfn {
 constexpr int kAsmThreads = 128;
+// general: every pair by the published formulas (okada.cuh), without the corner sums
 void launch_assemble_rect(cudaStream_t st, int64_t n_src, const double* src, int64_t n_recv, const double* recv,
-                          double G, double nu, double* Ks, double* Kn, int64_t ld, int layout);
+                          double G, double nu, double* Ks, double* Kn, int64_t ld, int layout, bool general = false);
 void launch_assemble_tri(cudaStream_t st, int64_t n_src, const double* P1, const double* P2, const double* P3,
                          const double* rake, int64_t n_recv, const double* centre, const double* nhat,
                          const double* shat, double G, double nu, double* Ks, double* Kn, int64_t ld, int layout);
