@@ -15,6 +15,7 @@
 #include "qdfn_internal.h"
 #include "hmat.cuh"
 #include "sim_device.cuh"
+#include "stage_ring.h"
 
 namespace qdfn {
 namespace {
@@ -323,7 +324,6 @@ __device__ __forceinline__ void red_fields(const unsigned long long* words, doub
 constexpr int kOpWarps = 8;                                     // operator role: warps [0, kOpWarps)
 constexpr int kOpThreads = kOpWarps * 32;
 constexpr int kProducerWarp = kSimThreads / 32 - 1;             // lane 0 fills the stage ring
-constexpr int kStages = 5;
 // FP32/BF16 steps that stream ahead: the solver warps [kOpWarps, kProducerWarp)
 // run the step's first reduction pass and its grid barrier on their own
 // (named barrier 1) while the operator warps and the producer finish the early
@@ -441,33 +441,30 @@ struct Pipe {
     uint64_t* full;
     uint64_t* empty;
     StageDesc* desc;
-    uint32_t cslot, cwrap;   // the next stage's slot and its round of the ring
+    RingPos take;            // where the next stage is taken from
     // producer (thread 0)
-    uint32_t filled, fslot, fwrap;   // stages filled; the next one's slot and its round of the ring
+    RingFill ring;
     long long ftile;         // tile being filled; -2 none yet, -1 no tiles left
     int fq, fnst, fseq;      // its next stage, its stage count, its sequence number
     int frb, fc, fj0, fleft; // its row block, column chunk, first column, columns not yet copied
     int64_t foff;            // byte offset of its next stage in both matrices
     int fphase, fnext;       // 0 this step's tiles, 1 the next step's, 2 done; the tile's step
     int fown;                // the block's own tile (StepCtx::own) is still to come
-    uint32_t last_stage[2];  // last stage of the latest tile using each x buffer
 };
-constexpr uint32_t kNoStage = 0xffffffffu;
 
 __device__ __forceinline__ void pipe_init(Pipe& pp, unsigned char* smem) {
     pp.stages = smem;
     pp.full = reinterpret_cast<uint64_t*>(smem + kPipeBytes);
     pp.empty = pp.full + kStages;
     pp.desc = reinterpret_cast<StageDesc*>(smem + kPipeBytes + kDescOffset);
-    pp.cslot = pp.cwrap = 0;
-    pp.filled = pp.fslot = pp.fwrap = 0;
+    pp.take = RingPos();
+    pp.ring = RingFill();
     pp.ftile = -2;
     pp.fq = pp.fnst = 0;
     pp.fseq = -1;
     pp.fphase = 0;
     pp.fnext = 0;
     pp.fown = 0;
-    pp.last_stage[0] = pp.last_stage[1] = kNoStage;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(pp.full + s, 1);
@@ -798,10 +795,9 @@ __device__ __forceinline__ bool produce_stage(const SimParams& p, Pipe& pp, type
     constexpr int VEC = M::VEC;
     constexpr int EB = kGranule / VEC;   // bytes per stored entry
     constexpr int64_t rows_per_blk = (int64_t)kOpThreads * VEC;
-    const uint32_t n = pp.filled;
-    const int slot = (int)pp.fslot;
+    const int slot = (int)pp.ring.at.slot;
     // the stage this slot held last must be released by every operator warp
-    if (pp.fwrap > 0 && !mbar_wait(pp.empty + slot, (pp.fwrap - 1) & 1u, kWaitLimitNs)) return false;
+    if (pp.ring.reused() && !mbar_wait(pp.empty + slot, pp.ring.at.phase() ^ 1u, kWaitLimitNs)) return false;
     if (pp.ftile == -2 || (pp.ftile >= 0 && pp.fq >= pp.fnst)) {
         int64_t nrb_reg, n_spec;
         spec_shape(p, nrb, &nrb_reg, &n_spec);
@@ -863,9 +859,8 @@ __device__ __forceinline__ bool produce_stage(const SimParams& p, Pipe& pp, type
     }
     StageDesc* d = pp.desc + slot;
     uint64_t* m = pp.full + slot;
-    pp.filled = n + 1;
-    if (++pp.fslot == (uint32_t)kStages) { pp.fslot = 0; ++pp.fwrap; }
     if (pp.ftile == -1) {              // end marker: completes the phase without bytes
+        pp.ring.advance();
         d->rb = -1;
         mbar_arrive(m);
         return true;
@@ -875,10 +870,8 @@ __device__ __forceinline__ bool produce_stage(const SimParams& p, Pipe& pp, type
     if (q == 0) {
         // the x buffer was last read by the tile before the previous one; its
         // last stage is released already unless that was within kStages stages
-        const uint32_t prev = pp.last_stage[xb];
-        if (prev != kNoStage && prev + kStages > n &&
-            !mbar_wait(pp.empty + (prev % kStages), (prev / kStages) & 1u, kWaitLimitNs))
-            return false;
+        const RingPos& last = pp.ring.last_at[xb];
+        if (pp.ring.x_in_use(xb) && !mbar_wait(pp.empty + last.slot, last.phase(), kWaitLimitNs)) return false;
     }
     const int nc = min(kColsPerStage, pp.fleft);
     reinterpret_cast<int4*>(d)[0] = make_int4(pp.frb, pp.fc, q, pp.fnst);
@@ -898,7 +891,8 @@ __device__ __forceinline__ bool produce_stage(const SimParams& p, Pipe& pp, type
         const X* xsrc = reinterpret_cast<const X*>(pp.fnext ? sc.xnext : sc.xcur);
         bulk_g2s(xs + (size_t)xb * p.xbuf, xsrc + (int64_t)pp.fj0 * R, xbytes, m, pol);
     }
-    if (q == pp.fnst - 1) pp.last_stage[xb] = n;
+    if (q == pp.fnst - 1) pp.ring.mark_last(xb);
+    pp.ring.advance();
     pp.fq = q + 1;
     pp.foff += bytes;
     pp.fleft -= nc;
@@ -923,9 +917,11 @@ __device__ bool produce_tiles(const SimParams& p, Pipe& pp, typename M::X* xs, c
     do {
         if (!produce_stage<M, R>(p, pp, xs, nrb, ntiles, pol, sc)) {
             atomicExch(p.gerr, QDFN_ERR_TIMEOUT);
-            const uint32_t from = pp.filled > (uint32_t)kStages ? pp.filled - kStages : 0u;
-            for (uint32_t k = from; k < pp.filled; ++k)
-                mbar_wait(pp.full + (k % kStages), (k / kStages) & 1u, kWaitLimitNs);
+            RingPos at = pp.ring.at;
+            for (int k = (int)min((uint64_t)kStages, pp.ring.filled); k > 0; --k) {
+                at.back();
+                mbar_wait(pp.full + at.slot, at.phase(), kWaitLimitNs);
+            }
             return false;
         }
     } while (pp.ftile != -1);
@@ -952,8 +948,8 @@ __device__ bool dense_matvec(const SimParams& p, Pipe& pp, typename M::X* xs, co
     int64_t i0 = 0;
     const X* xsb = xs;
     while (ok) {
-        const int slot = (int)pp.cslot;
-        if (!mbar_wait(pp.full + slot, pp.cwrap & 1u, kWaitLimitNs)) { ok = false; break; }
+        const int slot = (int)pp.take.slot;
+        if (!mbar_wait(pp.full + slot, pp.take.phase(), kWaitLimitNs)) { ok = false; break; }
         const StageDesc d = pp.desc[slot];
         if (d.q == 0 && d.rb >= 0) {   // a new tile
             i0 = (int64_t)d.rb * rows_per_blk + (int64_t)threadIdx.x * VEC;
@@ -1022,7 +1018,7 @@ __device__ bool dense_matvec(const SimParams& p, Pipe& pp, typename M::X* xs, co
         // every warp has arrived, the other warps run ahead into filled stages
         __syncwarp();
         if ((threadIdx.x & 31) == 0) mbar_arrive(pp.empty + slot);
-        if (++pp.cslot == (uint32_t)kStages) { pp.cslot = 0; ++pp.cwrap; }
+        pp.take.next();
         if (d.rb < 0) break;               // end marker
         if (d.q == d.nst - 1) {            // the tile is complete: publish its partials
             __threadfence();
