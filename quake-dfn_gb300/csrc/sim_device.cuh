@@ -361,9 +361,10 @@ static __device__ PatchOut solve_highv_pair(const PatchIn& p, double Dt, double 
 // A step below 1e-9 V ends the iteration, as in the reference (|VTest/V - 1|),
 // with an error of that step times the slope's error.
 // Returns false -- nothing decided -- when an operand or an iterate leaves the
-// ordinary range (V in (1e-25, 1e3), |ln(V/V0)| < 60) or 16 iterations are not
-// enough: the caller then runs the reference loop from the start, with all its
-// branches.
+// ordinary range (V in (1e-25, 1e3), |ln(V/V0)| < 60, g/a and the slope below
+// 1e30) or 16 iterations are not enough: the caller then runs the reference loop
+// from the start, with all its branches.  (FP32 overflows at 3e38, and __fdividef
+// returns 0 for divisors above 2^126: a step of 0 would pass for convergence.)
 // The solves are bound by the FP64 pipe (a warp instruction per 16 clocks and
 // SM) and the chain of dependent FP64 operations: ~110 of them per solve here,
 // ~620 in the secant loop.  Measured alone, 1 M patches on every SM: 1.41 ->
@@ -374,6 +375,9 @@ static __device__ PatchOut solve_highv_pair(const PatchIn& p, double Dt, double 
 // 2232 -> 1704 us.
 __device__ __forceinline__ bool hi_between(double x, double lo, double hi) {   // 0 < lo <= x < hi, NaN excluded
     return (unsigned)(__double2hiint(x) - __double2hiint(lo)) < (unsigned)(__double2hiint(hi) - __double2hiint(lo));
+}
+__device__ __forceinline__ bool hi_below(double x, double hi) {   // |x| < hi, NaN excluded
+    return (unsigned)(__double2hiint(x) & 0x7fffffff) < (unsigned)__double2hiint(hi);
 }
 __device__ __forceinline__ bool solve_lowv_newton(const PatchIn& p, double Dt, double eta, double alpha, int dr,
                                                   PatchOut& o) {
@@ -387,6 +391,7 @@ __device__ __forceinline__ bool solve_lowv_newton(const PatchIn& p, double Dt, d
     const double Fb = inv_sig * (p.K_Self * (p.TLD - fma(p.VOld, Dt, p.DispOld)) + p.tau0 - eta * p.VOld + p.dtau);
     const double g = inv_sig * (fma(p.K_Self, 0.5 * Dt, eta) + p.Mass * p.rDt);
     const double q = Dt * p.rDc, ga = g * p.ra, ba = p.b * p.ra;
+    if (!hi_below(ga, 1e30)) return false;
     const double c0 = (Fb - p.Friction0 - p.b * fm_log(th * (kV0 * p.rDc))) * p.ra;
     const float gaf = to_float(ga), qf = to_float(q), bqf = to_float(ba) * qf;
     double V = p.VOld;
@@ -395,10 +400,11 @@ __device__ __forceinline__ bool solve_lowv_newton(const PatchIn& p, double Dt, d
     for (;;) {
         ++it;
         const double x = fma(ba, fm_log(fma(V, q, 1.0)), fma(-ga, V - p.VOld, c0));
-        if (!((unsigned)(__double2hiint(x) & 0x7fffffff) < (unsigned)__double2hiint(60.0))) return false;
+        if (!hi_below(x, 60.0)) return false;
         const double e = fm_exp(x);
         const float f = to_float(fma(-kV0, e, V));
         const float slope = fmaf((float)kV0 * to_float(e), gaf - __fdividef(bqf, fmaf(Vf, qf, 1.f)), 1.f);
+        if (!(fabsf(slope) < 1e30f)) return false;
         const float d = __fdividef(f, slope);
         V -= to_double(d);
         if (!hi_between(V, 1e-25, 1e3)) return false;
@@ -609,7 +615,7 @@ __device__ __forceinline__ bool solve_highv_usual(const PatchIn& p, double Dt, d
     auto eval = [&](double V, double& Th, double& lv, double& lt, double& W) {
         if (!hi_between(V, 1e-27, 1e6)) return false;
         const double z = V * qn;
-        if (!((unsigned)(__double2hiint(z) & 0x7fffffff) < (unsigned)__double2hiint(600.0))) return false;
+        if (!hi_below(z, 600.0)) return false;
         const double ic = p.Dc * fm_rcp(V);
         Th = fma(p.ThetaOld - ic, fm_exp(z), ic);
         if (!hi_between(Th, 1e-30, 1e30)) return false;
@@ -626,8 +632,9 @@ __device__ __forceinline__ bool solve_highv_usual(const PatchIn& p, double Dt, d
         ++it;
         const double VTest = V, f = V - W;
         if (!eval(V + DV, Th2, l2, t2, W2)) return false;
-        const double fu = (V + DV) - W2;
-        V = VTest - f * DV * fm_rcp(fu - f);
+        const double df = (V + DV) - W2 - f;
+        if (!hi_below(df, 1e300)) return false;   // (fm_rcp's range)
+        V = VTest - f * DV * fm_rcp(df);
         if (!hi_between(V, 1e-27, 1e6) || !eval(V, Th, lv, lt, W)) return false;
         if (!(fabs(VTest - V) > kConv * V)) break;
         if (it >= 98) return false;
