@@ -409,6 +409,13 @@ int qdfn_apply_dense_noalloc(int64_t N, const double* Ks, const double* Kn, int6
  * division.  No counterpart in the reference (Julia's `/`). */
 int qdfn_check_division(int64_t n, const double* x, const double* d, double* q, void* stream);
 
+/* The kernels' own functions on DEVICE arrays, y[i] = f(x[i], d[i]), for
+ * arguments in their stated ranges; which: 0 logarithm, 1 exponential, 2
+ * reciprocal of the friction solves, 3 FP64 to FP32, 4 FP32 to FP64, 5 int32 to
+ * FP64; of the rectangle stiffness: 6 reciprocal, 7 the same corrected, 8 x/d,
+ * 9 square root, 10 its reciprocal.  d is read by 8 alone. */
+int qdfn_check_math(int which, int64_t n, const double* x, const double* d, double* y, void* stream);
+
 /* qdfn_assemble_rect_dev with every pair by the published formulas term by term
  * (scripts/Functions_OKADA3D.jl), where the assembly sums corner functions:
  * slower by a factor of five, and what its entries are compared with. */

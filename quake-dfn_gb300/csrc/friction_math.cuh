@@ -8,9 +8,11 @@
 // rest.  The FP64 pipe is this part's narrowest (a 64th of FP32), and an FP64
 // operation or a conversion between FP32 and FP64 takes ~62 clocks of a chain
 // and 16 of the SM's pipe, so the split is chosen to issue as few of both as
-// possible: the polynomial's terms whose FP32 rounding stays below 2^-55 of the
-// result are evaluated in FP32 beside the FP64 chain, and the conversions are
-// shifts and masks on the integer pipe.  In a chain (clocks): logarithm 560 and
+// possible: the polynomials' last terms are evaluated in FP32 beside the FP64
+// chain (their rounding is below 2^-55, absolute for the logarithm and relative
+// for the exponential), and the conversions are shifts and masks on the integer
+// pipe.  Errors: the logarithm's below 3 x 2^-53 of the result + 2^-55, the
+// exponential's below 1.3 x 2^-53 of it.  In a chain (clocks): logarithm 560 and
 // exponential 691 (681 and 872 with conversion instructions); CUDA's log 1936 and
 // exp 1650.
 #pragma once
@@ -37,8 +39,10 @@ __device__ __forceinline__ double to_double(int k) {
     return __hiloint2double(0x43300000, k ^ 0x80000000) - __hiloint2double(0x43300000, 0x80000000);
 }
 
-// 1/x to about an ulp, x normal: y (1 + e + e^2) from the hardware's estimate
-// (2^-20), e = 1 - x y
+// 1/x to about an ulp, x normal and 1/x normal.  With an estimate y and e = 1 - x y,
+// 1/x = y/(1 - e) = y (1 + e + e^2 + ...): the third-order member of Householder's
+// family (A. S. Householder, The Numerical Treatment of a Single Nonlinear
+// Equation, 1970), which leaves e^3 < 2^-60 of the hardware's 2^-20 estimate.
 __device__ __forceinline__ double fm_rcp(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

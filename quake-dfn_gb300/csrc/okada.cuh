@@ -88,7 +88,7 @@ __device__ __forceinline__ void acc9(double U[9], const double du[9], double DIS
 }
 
 // UA_V gradient rows (components 4..12 of the reference, here 0..8)
-__device__ void ua(double XI, double ET, double Q, double DISL1, double DISL2, double DISL3,
+static __device__ void ua(double XI, double ET, double Q, double DISL1, double DISL2, double DISL3,
                    const C0& c0, const C2& g, double U[9]) {
     const double ALP1 = c0.ALP1, ALP2 = c0.ALP2, SD = c0.SD, CD = c0.CD;
     const double XY = XI * g.Y11, QY = Q * g.Y11;
@@ -127,7 +127,7 @@ __device__ void ua(double XI, double ET, double Q, double DISL1, double DISL2, d
     acc9(U, du, DISL3);
 }
 
-__device__ void ub(double XI, double ET, double Q, double DISL1, double DISL2, double DISL3,
+static __device__ void ub(double XI, double ET, double Q, double DISL1, double DISL2, double DISL3,
                    const C0& c0, const C2& g, double U[9]) {
     const double ALP3 = c0.ALP3, SD = c0.SD, SDSD = c0.SDSD, SDCD = c0.SDCD;
     const double R = g.R, Y = g.Y, D = g.D;
@@ -189,7 +189,7 @@ __device__ void ub(double XI, double ET, double Q, double DISL1, double DISL2, d
 
 // UC_V: all twelve rows are needed because the image combination adds
 // DUC rows 1..3 into the z-gradient rows.
-__device__ void uc(double XI, double ET, double Q, double DISL1, double DISL2, double DISL3,
+static __device__ void uc(double XI, double ET, double Q, double DISL1, double DISL2, double DISL3,
                    double Z, const C0& c0, const C2& g, double U[12]) {
     const double ALP4 = c0.ALP4, ALP5 = c0.ALP5, SD = c0.SD, CD = c0.CD, SDSD = c0.SDSD,
                  CDCD = c0.CDCD, SDCD = c0.SDCD;
@@ -262,7 +262,7 @@ __device__ void uc(double XI, double ET, double Q, double DISL1, double DISL2, d
 }
 
 // Gradients g[0..8] = UXX,UYX,UZX,UXY,UYY,UZY,UXZ,UYZ,UZZ of Okada_DC3D_Vector.
-__device__ void dc3d_gradients(const C0& c0, double X, double Y, double Z, double DEPTH,
+static __device__ void dc3d_gradients(const C0& c0, double X, double Y, double Z, double DEPTH,
                                double AL1, double AL2, double AW1, double AW2, double DISL1,
                                double DISL2, double DISL3, double Ug[9]) {
     const double SD = c0.SD, CD = c0.CD;

@@ -65,13 +65,18 @@ QDFN_HD double rcp_est(double x) { return (double)(float)(1.0 / x); }
 QDFN_HD double rsqrt_est(double x) { return (double)(float)(1.0 / sqrt(x)); }
 #endif
 
-// 1/x to about an ulp: y (1 + e + e^2), e = 1 - x y (e^3 < 2^-60)
+// 1/x to about an ulp.  With an estimate y and e = 1 - x y, 1/x = y/(1 - e) =
+// y (1 + e + e^2 + ...): the third-order member of Householder's family (A. S.
+// Householder, The Numerical Treatment of a Single Nonlinear Equation, 1970);
+// e^3 < 2^-60.
 QDFN_HD double recip1(double x) {
     const double y = rcp_est(x), e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
 }
-// R = sqrt(R2) and 1/R: y (1 + e/2 + 3 e^2/8) with e = 1 - R2 y^2, then one
-// correction of R by its remainder
+// R = sqrt(R2) and 1/R: the same family's 1/sqrt(R2) = y (1 - e)^(-1/2) =
+// y (1 + e/2 + 3 e^2/8 + ...) with e = 1 - R2 y^2, then Newton's (Heron's) step
+// for the root, r + (R2 - r^2)/(2 r), whose remainder is exact in one fused
+// operation.
 QDFN_HD void root(double R2, double& R, double& i1) {
     const double y = rsqrt_est(R2), e = fma(-(R2 * y), y, 1.0);
     i1 = fma(y * e, fma(e, 0.375, 0.5), y);
@@ -114,13 +119,14 @@ struct Src {
 QDFN_HD bool is_steep(double CD) { return CD != 0.0 && fabs(CD) < 0.1; }
 
 // 1/x, correctly rounded but for rare ties (recip1 rounds otherwise one time in
-// a hundred)
+// a hundred): Newton's step from a value within an ulp (Markstein 1990, cited at
+// div_by in sim_device.cuh)
 QDFN_HD double recip2(double x) {
     const double y = recip1(x);
     return fma(fma(-x, y, 1.0), y, y);
 }
-// x/d, correctly rounded but for rare ties: i = 1/d to about an ulp, then the
-// quotient corrected by its remainder
+// x/d, correctly rounded but for rare ties: i = 1/d to about an ulp, then
+// Markstein's correction of the quotient by its remainder
 QDFN_HD double quotient(double x, double d, double i) {
     const double q = x * i;
     return fma(fma(-q, d, x), i, q);
