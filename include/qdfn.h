@@ -416,6 +416,15 @@ int qdfn_check_division(int64_t n, const double* x, const double* d, double* q, 
  * 9 square root, 10 its reciprocal.  d is read by 8 alone. */
 int qdfn_check_math(int which, int64_t n, const double* x, const double* d, double* y, void* stream);
 
+/* One solver of the step loop on n patches (DEVICE arrays, row-major): which: 0
+ * the short low-velocity solve, 1 the short high-velocity one, 2 and 3 the
+ * reference's secant loops (low, high) on one lane, 4 and 5 on a lane pair.  in
+ * [n][17]: slip, friction, theta, V, F0, a, b, Dc, K_self, Omega, mass, sigma, TLD,
+ * dtau, old sigma, tau0, Dt.  out [n][10]: 1 or (0, 1: operands left to the loops) 0,
+ * V, friction, slip, theta, Dt, instability, flag, iterations, error. */
+int qdfn_check_solve(int which, int64_t n, const double* in, double eta, double alpha, int evolution_dr,
+                     double switch_v, double* out, void* stream);
+
 /* qdfn_assemble_rect_dev with every pair by the published formulas term by term
  * (scripts/Functions_OKADA3D.jl), where the assembly sums corner functions:
  * slower by a factor of five, and what its entries are compared with. */

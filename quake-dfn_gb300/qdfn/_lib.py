@@ -35,6 +35,7 @@ EXPORTS = [
     "qdfn_ensemble_create", "qdfn_ensemble_destroy", "qdfn_ensemble_get_blocks", "qdfn_ensemble_set_blocks",
     "qdfn_ensemble_balance", "qdfn_ensemble_run", "qdfn_ensemble_run_async", "qdfn_ensemble_sync",
     "qdfn_ensemble_shares", "qdfn_ensemble_set_fill", "qdfn_check_division", "qdfn_check_rect", "qdfn_check_math",
+    "qdfn_check_solve",
     "qdfn_adjoint_run",
     "qdfn_assemble_tri_pairs_dev", "qdfn_set_early_cols", "qdfn_get_early_cols",
     "qdfn_ensemble_state_bytes", "qdfn_ensemble_set_state_all", "qdfn_ensemble_get_state_all",
@@ -141,6 +142,8 @@ def load():
     L.qdfn_ensemble_set_state_all.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     L.qdfn_ensemble_get_state_all.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int]
     L.qdfn_check_math.argtypes = [C.c_int, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    L.qdfn_check_solve.argtypes = [C.c_int, C.c_int64, C.c_void_p, C.c_double, C.c_double, C.c_int, C.c_double,
+                                   C.c_void_p, C.c_void_p]
     L.qdfn_check_rect.argtypes = L.qdfn_assemble_rect_dev.argtypes
     L.qdfn_check_division.argtypes = [C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     L.qdfn_assemble_tri_pairs_dev.argtypes = [C.c_int64] + [C.c_void_p] * 9 + [C.c_double, C.c_double] + \
