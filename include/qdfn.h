@@ -362,8 +362,9 @@ int qdfn_get_kself(const qdfn_ctx* ctx, double* kself);
  * :26-182, the products at scripts/Functions_RSFDFN3DMain_D.jl:199-202 and the
  * time-step control at :162-201).
  *
- * Runs nsteps steps from the context's current state (one step per launch,
- * checkpointing the state every checkpoint_every steps; 0 = ceil(sqrt(nsteps))),
+ * Runs nsteps steps from the context's current state (a launch per
+ * checkpoint_every steps, with the state kept before each; 0 =
+ * ceil(sqrt(nsteps))),
  * then sweeps them backwards: per step the implicit-function derivative of each
  * patch's converged solve, the transposed products E^T and Kn^T over the stored
  * operator (its precision), and the time step's derivative through the patch
@@ -376,7 +377,9 @@ int qdfn_get_kself(const qdfn_ctx* ctx, double* kself);
  * seed_dT[k] to that of its time T, after step seed_step[k] (0 = the starting
  * state, nsteps = the last), e.g. the derivatives of an event onset time
  * interpolated between two steps.  Outputs dL_da, dL_db, dL_dDc are
- * [n_inst][N] host arrays.  Needs a dense operator and Alpha_Evo = 0. */
+ * [n_inst][N] host arrays.  Needs a dense operator and Alpha_Evo = 0.
+ * timeout_s bounds the wall time of a step (0 = no bound): a launch of k steps
+ * ends with QDFN_ERR_TIMEOUT after k times as long. */
 int qdfn_adjoint_run(qdfn_ctx* ctx, int64_t nsteps, int64_t checkpoint_every, const double* dL_dD_final,
                      int64_t n_seeds, const int64_t* seed_step, const int32_t* seed_inst,
                      const int64_t* seed_patch, const double* seed_dV, const double* seed_dD,

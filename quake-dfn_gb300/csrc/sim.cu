@@ -766,7 +766,10 @@ extern "C" int qdfn_adjoint_run(qdfn_ctx* c, int64_t nsteps, int64_t checkpoint_
     int64_t cp = checkpoint_every > 0 ? checkpoint_every : (int64_t)std::ceil(std::sqrt((double)nsteps));
     cp = std::max<int64_t>(1, std::min(cp, nsteps));
     const int64_t nseg = (nsteps + cp - 1) / cp;
-    const uint64_t budget_ns = (uint64_t)((timeout_s > 0 ? timeout_s : 1e6) * 1e9);
+    // timeout_s is a step's, whatever the segments: a launch has its steps' together
+    // (at most 30 years, which the deadline can hold)
+    const double step_s = timeout_s > 0 ? timeout_s : 1e6;
+    auto budget_ns = [&](int64_t steps) { return (uint64_t)(std::min(step_s * (double)steps, 1e9) * 1e9); };
     cudaStream_t st = nullptr;
     int rc;
     // checkpoints (nseg, the state before each segment) and the final state
@@ -800,7 +803,8 @@ extern "C" int qdfn_adjoint_run(qdfn_ctx* c, int64_t nsteps, int64_t checkpoint_
     // ---- forward: a checkpoint before each segment
     for (int64_t seg = 0; seg < nseg; ++seg) {
         if ((rc = snap_save(c, ck[seg], st))) return rc;
-        if ((rc = launch_steps(c, std::min(cp, nsteps - seg * cp), budget_ns, nullptr, st))) return rc;
+        const int64_t len = std::min(cp, nsteps - seg * cp);
+        if ((rc = launch_steps(c, len, budget_ns(len), nullptr, st))) return rc;
         if ((rc = run_status(c, st))) return rc;
     }
     if ((rc = snap_save(c, ck[nseg], st))) return rc;
@@ -849,7 +853,7 @@ extern "C" int qdfn_adjoint_run(qdfn_ctx* c, int64_t nsteps, int64_t checkpoint_
         QDFN_CUDA(cudaMemcpyAsync(tp.A, s6 + 4 * RN, RN * 8, cudaMemcpyDeviceToDevice, st));
         QDFN_CUDA(cudaMemcpyAsync(tp.T, ck[seg].Tdt, Rk * 8, cudaMemcpyDeviceToDevice, st));
         QDFN_CUDA(cudaMemcpyAsync(tp.dt, ck[seg].Tdt + Rk, Rk * 8, cudaMemcpyDeviceToDevice, st));
-        if ((rc = launch_steps(c, len, budget_ns, &tp, st))) return rc;
+        if ((rc = launch_steps(c, len, budget_ns(len), &tp, st))) return rc;
         if ((rc = run_status(c, st))) return rc;
         for (int64_t t = len; t >= 1; --t) {   // the step taking tape state t-1 to t
             AdjLocalArgs a{};
