@@ -304,8 +304,8 @@ int qdfn_ensemble_shares(int n, const double* cost, int nsm, int* out);
 /* Cumulative device counters of the context's runs (first n of): ns spent in
  * [0] time-step control, [1] elastic operator, [2] friction solves and retries,
  * [3] state rotation; [4] solve passes (1 + retries per step), [5] steps;
- * [6] low-velocity patch solves, [7] their secant iterations, [8] high-velocity
- * patch solves, [9] their secant iterations (summed over patches, instances
+ * [6] low-velocity patch solves, [7] their iterations, [8] high-velocity
+ * patch solves, [9] their iterations (summed over patches, instances
  * (padding instances included) and solve passes); [10] ns of [2] that the
  * first block spent on its own solves and block reduction, [11] ns of [2] it
  * waited at the grid barrier after them; [12]/[13] ns the first block's

@@ -183,7 +183,7 @@ k_assemble_rect(int64_t n_src, const double* __restrict__ src, int64_t n_recv,
 }  // namespace
 
 // Sources per block and turn: a turn costs a thread ~250 FP64 operations of its
-// receiver's and sources' sines and cosines beside ~1,340 per pair, so 8 where
+// receiver's and sources' sines and cosines beside ~1,400 per pair, so 8 where
 // that still leaves four rounds of the GPU's resident blocks (two per SM at 255
 // registers), down to 1 for small calls, where every pair starts at once.
 void launch_assemble_rect(cudaStream_t st, int64_t n_src, const double* src, int64_t n_recv, const double* recv,

@@ -73,7 +73,7 @@ __device__ __forceinline__ void stiffness(const Medium& m, const tdhs::TriRecv& 
 // triangles on one, their images on the next, the sides on the third.  Bound by
 // the FP64 pipe (~8,000 operations a pair; 43,500 with the published formulas'
 // divisions and every constant formed per pair): 1,100 x 1,100 triangles 138.9 ->
-// 20.7 ms.
+// 21.1 ms.
 __global__ void __launch_bounds__(kAsmThreads)
 k_assemble_tri(int64_t n_src, const double* __restrict__ P1, const double* __restrict__ P2,
                const double* __restrict__ P3, const double* __restrict__ rake, int64_t n_recv,

@@ -11,7 +11,8 @@
 // components are formed once from the sums, where okada.cuh forms every
 // component at every corner for three slip directions (opening is zero here).
 // The kernel is bound by the FP64 pipe, so what counts is the number of FP64
-// operations: ~1,340 per pair against ~7,500 (no divisions either: one
+// operations: ~1,470 per pair of a fault network against ~7,540 (ncu, the
+// source's and receiver's constants included; no divisions either: one
 // reciprocal square root per corner gives R and 1/R, and 1/(R + xi),
 // 1/(R + eta), 1/(R + D~) are reciprocals by Newton's iteration from the
 // hardware's estimate).

@@ -270,7 +270,8 @@ int configure_launch(qdfn_ctx* c) {
         };
         int64_t clen = chunk(tiles_per_sm, fp64);
         // one tile only where both splits end on the groups of 32 columns that FP32
-        // products are summed in: the results are the same
+        // products are summed in: then the same FP32 sums are gathered, in error-free
+        // pairs, in another order (about 2^-48 of a row's sum)
         if (!fp64 && !tiles_env && one <= 384 && clen % 32 == 0) clen = chunk(1, true);
         c->chunk_len = clen;
         c->nchunk = (int)((c->N + clen - 1) / clen);
@@ -978,12 +979,9 @@ void ensemble_detach(qdfn_ensemble* e, qdfn_ctx* c) {
 
 // Estimated SM-nanoseconds of one step of a member on one SM: its operator
 // bytes at one SM's share of the HBM stream (~44 B/ns) plus 450 ns per patch
-// solve.  Only the starting point of the split; qdfn_ensemble_balance re-divides
-// by measured time.  (A solve takes ~85 ns of an SM by now, beside the stream:
-// max(bytes / 44, 85 per solve) starts as the balanced split does, 40 networks x
-// 4, 15 steps 4.57 -> 4.45 ms.  But the shares set the column chunks, and with
-// them the groups of 32 columns that FP32 products are summed in: the results
-// would move by that rounding, 2e-8 of the largest acceleration.)
+// solve (85 ns by now, beside the stream).  Only the starting point of the split;
+// qdfn_ensemble_balance re-divides by measured time.  Another estimate gives other
+// column chunks and with them other roundings of the FP32 products.
 double member_cost(const qdfn_ctx* c) {
     const double esz = c->prec == QDFN_FP64 ? 8.0 : 4.0;
     const double n = (double)c->N;

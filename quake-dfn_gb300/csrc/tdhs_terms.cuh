@@ -15,6 +15,10 @@
 // The stresses are differences of large terms, so the formulas' own rounding
 // error is 1e-9 of Kn over a near-field block (113-bit arithmetic as the value),
 // as published and here alike (6.46e-9 and 6.45e-9); the two differ by 2e-11.
+// Over far blocks (18 x 18 triangles, 0.6 to 8 km off, geometric mean of the
+// 2-norm of the error and of the difference) 1.5e-11 and 8e-12 at dips of 70
+// degrees, 4e-10 and 1.3e-10 at 85: a side near the vertical multiplies either by
+// up to cot^2 of its angle to it, 1.6e-7 and 3e-8 at 89.67 degrees.
 #pragma once
 #include "qdfn_internal.h"
 
